@@ -185,16 +185,16 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    // The whole warp walks the tiles, one elected lane issues (see elect_one).
+    {
       const uint32_t idesc_qk = umma_instr_desc(1, 1, 1, 0, 0, 128, 128);   // A, B K-major
       // A (P) and B (V) must have the same 16-bit format: kind::f16 with an f16 A and a bf16 B operand
       // raises an illegal-instruction fault on sm_100a, so P is rounded to bf16 like V
       const uint32_t idesc_pv = umma_instr_desc(1, 1, 1, 0, 1, 128, 128);   // B (V) MN-major
       const int nt[2] = {n0, n1};
       int err = 0;
-      // This thread's instruction stream is the tensor pipe's critical path: descriptors are split into
-      // a constant high word and a low word (start address in 16-byte units | leading offset << 16)
-      // that advances by a compile-time constant per K step.
+      // Descriptors are split into a constant high word and a low word (start address in 16-byte units |
+      // leading offset << 16) that advances by a compile-time constant per K step.
       const uint32_t hi_k = uint32_t(umma_smem_desc(0, 16, 1024) >> 32);
       const uint32_t hi_v = uint32_t(umma_smem_desc(0, 16384, 1024) >> 32);
       auto lo_k = [](uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); };
@@ -209,22 +209,25 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       auto issue_qk = [&](int t, uint32_t kslot) {
         const uint32_t d = tmem + uint32_t(t) * 128u;
         const uint32_t a = q_lo[t], b = lo_k(kslot);
+        if (elect_one()) {
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
-          umma_f16(d, dsc(a + off, hi_k), dsc(b + off, hi_k), idesc_qk, s > 0 ? 1u : 0u);
+          for (int s = 0; s < 8; ++s) {
+            const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
+            umma_f16(d, dsc(a + off, hi_k), dsc(b + off, hi_k), idesc_qk, s > 0 ? 1u : 0u);
+          }
+          umma_commit(s_full_b[t]);
         }
-        umma_commit(s_full_b[t]);
+        __syncwarp();
       };
       // ring position of the next entry to consume (same order as the producer fills it)
       int slot = 0;
       uint32_t ph = 0;
-      auto ring_wait = [&]() { return mbar_wait(smem_u32(&bars->kv_full[slot]), ph); };
+      auto ring_wait = [&]() { return mbar_wait_warp(smem_u32(&bars->kv_full[slot]), ph); };
       auto ring_release = [&]() {
-        umma_commit(smem_u32(&bars->kv_empty[slot]));   // free once the MMAs issued so far retire
+        if (elect_one()) umma_commit(smem_u32(&bars->kv_empty[slot]));   // free once the MMAs issued so far retire
         if (++slot == kRing) { slot = 0; ph ^= 1u; }
       };
-      if (!mbar_wait(smem_u32(&bars->q_full), 0)) err = ERR_WAIT_FULL;
+      if (!mbar_wait_warp(smem_u32(&bars->q_full), 0)) err = ERR_WAIT_FULL;
       if (!err && !ring_wait()) err = ERR_WAIT_FULL;
       if (!err) {
         tc_fence_after();
@@ -239,7 +242,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const uint32_t kslot = ring_s + uint32_t(slot) * kSlot;
           for (int t = 0; t < 2 && !err; ++t) {
             if (j + 1 >= nt[t]) continue;
-            if (!mbar_wait(s_free_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
+            if (!mbar_wait_warp(s_free_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
             tc_fence_after();
             issue_qk(t, kslot);
           }
@@ -251,21 +254,24 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t v_lo = lo_v(ring_s + uint32_t(slot) * kSlot);
         for (int t = 0; t < 2 && !err; ++t) {
           if (j >= nt[t]) continue;
-          if (!mbar_wait(p_ready_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
+          if (!mbar_wait_warp(p_ready_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
           tc_fence_after();
           const uint32_t d = tmem + 256u + uint32_t(t) * 128u;
           const uint32_t a = p_lo[t];
+          if (elect_one()) {
 #pragma unroll
-          for (int s = 0; s < 8; ++s) {
-            const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
-            umma_f16(d, dsc(a + off, hi_k), dsc(v_lo + uint32_t(s) * 128u, hi_v), idesc_pv, (j > 0 || s > 0) ? 1u : 0u);
+            for (int s = 0; s < 8; ++s) {
+              const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
+              umma_f16(d, dsc(a + off, hi_k), dsc(v_lo + uint32_t(s) * 128u, hi_v), idesc_pv, (j > 0 || s > 0) ? 1u : 0u);
+            }
+            umma_commit(pv_full_b[t]);
           }
-          umma_commit(pv_full_b[t]);
+          __syncwarp();
         }
         if (err) break;
         ring_release();
       }
-      if (err) atomicExch(p.error, err);
+      if (err && lane == 0) atomicExch(p.error, err);
     }
   } else {
     // ---------------------------------------------------------------- softmax / epilogue

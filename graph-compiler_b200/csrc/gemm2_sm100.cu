@@ -151,11 +151,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (even CTA)
-    if (lane == 0 && rank == 0) {
-      // The issuing thread is alone in its warp, so every instruction it executes is on the tensor
-      // pipe's critical path: descriptors are built once and advanced with one 32-bit add per MMA
-      // (the start-address field is the low 14 bits, in 16-byte units), and the ring position is
-      // carried in counters instead of being derived with divisions.
+    // The whole warp walks the loop, one elected lane issues (see elect_one).  Descriptors are built once and advanced
+    // with one 32-bit add per MMA (the start-address field is the low 14 bits, in 16-byte units), and the ring position
+    // is carried in counters instead of being derived with divisions.
+    if (rank == 0) {
       const uint64_t adesc0 = umma_smem_desc(base, p.a.lbo, p.a.sbo);
       const uint64_t bdesc0 = umma_smem_desc(base + p.a.bytes, p.b.lbo, p.b.sbo);
       const uint32_t a_hi = uint32_t(adesc0 >> 32), b_hi = uint32_t(bdesc0 >> 32);
@@ -168,38 +167,40 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int s = 0;
       uint32_t ph = 0;
       int err = 0;
-      if (p.wait_counter != nullptr && !pair_rows_landed(p)) err = ERR_WAIT_PEER;
+      if (p.wait_counter != nullptr && !__all_sync(0xFFFFFFFFu, pair_rows_landed(p))) err = ERR_WAIT_PEER;
       for (int u = pair; u < units && !err; u += pairs, ++tcount) {
         const int tile = u / p.splits, split = u - tile * p.splits;
         const int kb0 = split * kb_per_split, kb1 = min(p.k_blocks, kb0 + kb_per_split);
         const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&bars->tmem_empty[acc]), acc_ph ^ 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
+        if (!mbar_wait_warp(smem_u32(&bars->tmem_empty[acc]), acc_ph ^ 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * uint32_t(p.BN);
         uint32_t accum = 0;   // the first MMA of a tile overwrites the accumulator (zero-init at the first K block)
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(smem_u32(&bars->full[s]), ph)) { err = ERR_WAIT_FULL; break; }
+          if (!mbar_wait_warp(smem_u32(&bars->full[s]), ph)) { err = ERR_WAIT_FULL; break; }
           tc_fence_after();
           const uint32_t al = a_lo0 + uint32_t(s) * stage_step, bl = b_lo0 + uint32_t(s) * stage_step;
-          if (KIND == 0) {
-            umma_f16_pair(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accum);
-            umma_f16_pair(d_tmem, desc(al + a_k, a_hi), desc(bl + b_k, b_hi), idesc, 1u);
-            umma_f16_pair(d_tmem, desc(al + 2 * a_k, a_hi), desc(bl + 2 * b_k, b_hi), idesc, 1u);
-            umma_f16_pair(d_tmem, desc(al + 3 * a_k, a_hi), desc(bl + 3 * b_k, b_hi), idesc, 1u);
-          } else {
-            umma_i8_pair(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accum);
-            umma_i8_pair(d_tmem, desc(al + a_k, a_hi), desc(bl + b_k, b_hi), idesc, 1u);
-            umma_i8_pair(d_tmem, desc(al + 2 * a_k, a_hi), desc(bl + 2 * b_k, b_hi), idesc, 1u);
-            umma_i8_pair(d_tmem, desc(al + 3 * a_k, a_hi), desc(bl + 3 * b_k, b_hi), idesc, 1u);
+          if (elect_one()) {
+            if (KIND == 0) {
+              umma_f16_pair(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accum);
+              umma_f16_pair(d_tmem, desc(al + a_k, a_hi), desc(bl + b_k, b_hi), idesc, 1u);
+              umma_f16_pair(d_tmem, desc(al + 2 * a_k, a_hi), desc(bl + 2 * b_k, b_hi), idesc, 1u);
+              umma_f16_pair(d_tmem, desc(al + 3 * a_k, a_hi), desc(bl + 3 * b_k, b_hi), idesc, 1u);
+            } else {
+              umma_i8_pair(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accum);
+              umma_i8_pair(d_tmem, desc(al + a_k, a_hi), desc(bl + b_k, b_hi), idesc, 1u);
+              umma_i8_pair(d_tmem, desc(al + 2 * a_k, a_hi), desc(bl + 2 * b_k, b_hi), idesc, 1u);
+              umma_i8_pair(d_tmem, desc(al + 3 * a_k, a_hi), desc(bl + 3 * b_k, b_hi), idesc, 1u);
+            }
+            umma_commit_pair(smem_u32(&bars->empty[s]));   // stage reusable once these MMAs retire
+            if (kb + 1 == kb1) umma_commit_pair(smem_u32(&bars->tmem_full[acc]));   // accumulator complete
           }
+          __syncwarp();
           accum = 1u;
-          umma_commit_pair(smem_u32(&bars->empty[s]));   // stage reusable once these MMAs retire
           if (++s == stages) { s = 0; ph ^= 1u; }
         }
-        if (err) break;
-        umma_commit_pair(smem_u32(&bars->tmem_full[acc])); // accumulator complete
       }
-      if (err) atomicExch(p.error, err);
+      if (err && lane == 0) atomicExch(p.error, err);
     }
   } else if (warp < 6) {
     // ------------------------------------------------------------------ epilogue (both CTAs)

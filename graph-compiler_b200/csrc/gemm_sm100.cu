@@ -178,38 +178,37 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      // The issuing thread is alone in its warp, so every instruction it executes is on the tensor
-      // pipe's critical path: descriptors are built once and advanced with one 32-bit add per MMA
-      // (the start-address field is the low 14 bits, in 16-byte units), and the ring position is
-      // carried in counters instead of being derived with divisions.
-      const uint64_t adesc0 = umma_smem_desc(base, p.a.lbo, p.a.sbo);
-      const uint64_t bdesc0 = umma_smem_desc(base + p.a.bytes, p.b.lbo, p.b.sbo);
-      const uint32_t a_hi = uint32_t(adesc0 >> 32), b_hi = uint32_t(bdesc0 >> 32);
-      const uint32_t a_lo0 = uint32_t(adesc0), b_lo0 = uint32_t(bdesc0);
-      const uint32_t stage_step = stage_bytes >> 4, a_k = p.a.kstep >> 4, b_k = p.b.kstep >> 4;
-      const uint32_t a_sub = p.a.sub_step >> 4, b_sub = p.b.sub_step >> 4;   // next K block inside a stage
-      const int kpb = max(p.kpb, 1);
-      const uint32_t idesc = p.idesc;
-      const int stages = p.stages;
-      auto desc = [](uint32_t lo, uint32_t hi) { return (uint64_t(hi) << 32) | uint64_t(lo); };
-      uint32_t tcount = 0;
-      int s = 0;
-      uint32_t ph = 0;
-      int err = 0;
-      if (p.wait_counter != nullptr && !peer_rows_landed(p)) err = ERR_WAIT_PEER;
-      for (int u = blockIdx.x; u < units && !err; u += gridDim.x, ++tcount) {
-        const int tile = u / p.splits, split = u - tile * p.splits;
-        const int kb0 = split * kb_per_split, kb1 = min(p.k_blocks, kb0 + kb_per_split);
-        const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&bars->tmem_empty[acc]), acc_ph ^ 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
+    // The whole warp walks the loop, one elected lane issues (see elect_one).  Descriptors are built once and advanced
+    // with one 32-bit add per MMA (the start-address field is the low 14 bits, in 16-byte units), and the ring position
+    // is carried in counters instead of being derived with divisions.
+    const uint64_t adesc0 = umma_smem_desc(base, p.a.lbo, p.a.sbo);
+    const uint64_t bdesc0 = umma_smem_desc(base + p.a.bytes, p.b.lbo, p.b.sbo);
+    const uint32_t a_hi = uint32_t(adesc0 >> 32), b_hi = uint32_t(bdesc0 >> 32);
+    const uint32_t a_lo0 = uint32_t(adesc0), b_lo0 = uint32_t(bdesc0);
+    const uint32_t stage_step = stage_bytes >> 4, a_k = p.a.kstep >> 4, b_k = p.b.kstep >> 4;
+    const uint32_t a_sub = p.a.sub_step >> 4, b_sub = p.b.sub_step >> 4;   // next K block inside a stage
+    const int kpb = max(p.kpb, 1);
+    const uint32_t idesc = p.idesc;
+    const int stages = p.stages;
+    auto desc = [](uint32_t lo, uint32_t hi) { return (uint64_t(hi) << 32) | uint64_t(lo); };
+    uint32_t tcount = 0;
+    int s = 0;
+    uint32_t ph = 0;
+    int err = 0;
+    if (p.wait_counter != nullptr && !__all_sync(0xFFFFFFFFu, peer_rows_landed(p))) err = ERR_WAIT_PEER;
+    for (int u = blockIdx.x; u < units && !err; u += gridDim.x, ++tcount) {
+      const int tile = u / p.splits, split = u - tile * p.splits;
+      const int kb0 = split * kb_per_split, kb1 = min(p.k_blocks, kb0 + kb_per_split);
+      const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
+      if (!mbar_wait_warp(smem_u32(&bars->tmem_empty[acc]), acc_ph ^ 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * uint32_t(p.BN);
+      uint32_t accum = 0;   // the first MMA of a tile overwrites the accumulator (zero-init at the first K block)
+      for (int kb = kb0; kb < kb1; kb += kpb) {
+        if (!mbar_wait_warp(smem_u32(&bars->full[s]), ph)) { err = ERR_WAIT_FULL; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * uint32_t(p.BN);
-        uint32_t accum = 0;   // the first MMA of a tile overwrites the accumulator (zero-init at the first K block)
-        for (int kb = kb0; kb < kb1; kb += kpb) {
-          if (!mbar_wait(smem_u32(&bars->full[s]), ph)) { err = ERR_WAIT_FULL; break; }
-          tc_fence_after();
-          uint32_t al = a_lo0 + uint32_t(s) * stage_step, bl = b_lo0 + uint32_t(s) * stage_step;
+        uint32_t al = a_lo0 + uint32_t(s) * stage_step, bl = b_lo0 + uint32_t(s) * stage_step;
+        if (elect_one()) {
 #pragma unroll 1
           for (int sub = 0; sub < kpb; ++sub, al += a_sub, bl += b_sub) {
             if (KIND == 0) {
@@ -225,15 +224,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
             accum = 1u;
           }
-          accum = 1u;
           umma_commit(smem_u32(&bars->empty[s]));   // stage reusable once these MMAs retire
-          if (++s == stages) { s = 0; ph ^= 1u; }
+          if (kb + kpb >= kb1) umma_commit(smem_u32(&bars->tmem_full[acc]));   // accumulator complete
         }
-        if (err) break;
-        umma_commit(smem_u32(&bars->tmem_full[acc])); // accumulator complete
+        __syncwarp();
+        accum = 1u;
+        if (++s == stages) { s = 0; ph ^= 1u; }
       }
-      if (err) { atomicExch(p.error, err); bars->abort_flag = 1; }
     }
+    if (err && lane == 0) { atomicExch(p.error, err); bars->abort_flag = 1; }
   } else if (warp < 6) {
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM lane quadrant this warp may read

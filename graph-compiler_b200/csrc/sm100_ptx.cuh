@@ -58,6 +58,27 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
+// One lane of a converged warp (the same one every time).  The single-thread instructions of an MMA or copy warp are
+// issued under this predicate, with the loop around them run by the WHOLE warp: their operands then live in uniform
+// registers.  Under `if (lane == 0)` every tcgen05.mma first moves its descriptors there one by one - measured on the
+// CTA-pair kernel 640 cycles per K block against 518 in this form (the tensor pipe needs 512).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
+// Bounded wait of a whole, converged warp; the answer is the same in every lane, so the warp stays together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  if (__all_sync(0xFFFFFFFFu, mbar_test(bar, parity))) return true;
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 256; ++i)
+      if (__all_sync(0xFFFFFFFFu, mbar_test(bar, parity))) return true;
+    if (__any_sync(0xFFFFFFFFu, clock64() - t0 > WAIT_LIMIT_CYCLES)) return false;
+  }
+}
+
 // ----------------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
