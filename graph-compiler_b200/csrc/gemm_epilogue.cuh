@@ -319,14 +319,48 @@ __device__ __forceinline__ void gemm_epilogue_tail(const GemmParams &p, uint32_t
 // raw f32 / s32 planes).
 // Each thread owns one accumulator row: TMEM -> registers -> rounding and post-ops on packed pairs ->
 // 16-byte chunks into a swizzled 32 x 128-byte staging slab -> one cp.async.bulk.tensor store per slab
-// issued by lane 0.  Two staging slabs per warp alternate, so the copy engine drains one while the
+// issued by one lane.  Two staging slabs per warp alternate, so the copy engine drains one while the
 // warp fills the other; rows and columns beyond the output are clipped by the copy engine.
+// One warp per scheduler runs this, so it is bound by its own instruction stream and nothing overlaps the last tile of
+// a CTA: the post-ops are compile-time choices, packed two columns to an instruction, without a branch per element
+// (NaN patch: one test per slab).  Measured per 128 x 256 bf16 tile with its stores: 12000 cycles with a branch and
+// unpacked arithmetic per element, 4900 in this form.
+enum EpiMode : int { EPI_RAW = 0, EPI_BF16 = 1, EPI_BF16_BIAS = 2, EPI_DEQUANT = 3 };
+
+__device__ __forceinline__ int epilogue_mode(const GemmParams &p) {
+  return p.out_kind == OUT_BF16 ? (p.bias_kind == BIAS_BF16 ? EPI_BF16_BIAS : EPI_BF16) : p.out_kind == OUT_DEQUANT_F32 ? EPI_DEQUANT : EPI_RAW;
+}
+
+// This lane's share of a slab's per-column operands: the bias pair of columns col0 + 2 lane, + 1 (bf16), or scale / bias /
+// compensation of column col0 + lane (dequantisation).  Loaded one slab ahead - the first one before the accumulator is
+// waited for - and handed round by shuffles: loaded at the point of use they cost 400 cycles a slab.
+struct EpiColumns {
+  uint32_t bias = 0, scale = 0, comp = 0;
+};
+__device__ __forceinline__ EpiColumns epilogue_columns(const GemmParams &p, int col0, int lane) {
+  EpiColumns e;
+  if (p.bias_kind == BIAS_BF16) {
+    const uint16_t *b = reinterpret_cast<const uint16_t *>(p.bias);
+    const int c = col0 + 2 * lane;
+    if (c < p.out_cols) e.bias = b[c];
+    if (c + 1 < p.out_cols) e.bias |= uint32_t(b[c + 1]) << 16;
+  } else if (p.out_kind == OUT_DEQUANT_F32) {
+    const int c = col0 + lane;
+    if (c < p.out_cols) {
+      e.scale = __float_as_uint(p.scale[c]);
+      if (p.bias_kind == BIAS_F32) e.bias = reinterpret_cast<const uint32_t *>(p.bias)[c];
+      if (p.comp) e.comp = uint32_t(p.comp[c]);
+    }
+  }
+  return e;
+}
+
 // stg: this warp's two 4 KiB slabs (1 KiB aligned); buf: slab to fill next (kept by the caller across tiles).
-template <int KIND>
-__device__ __forceinline__ void gemm_epilogue_tile_tma(const GemmParams &p, uint32_t t_addr, int row0, int nn0, int split,
-                                                       int q, int lane, uint8_t *stg, uint32_t &buf) {
-  const bool two_byte = (p.out_kind == OUT_BF16);
-  const int slab_cols = two_byte ? 64 : 32;
+template <int KIND, int MODE, bool RELU>
+__device__ __forceinline__ void epilogue_tile_tma(const GemmParams &p, uint32_t t_addr, int row0, int nn0, int split,
+                                                  int q, int lane, uint8_t *stg, uint32_t &buf, EpiColumns cols) {
+  constexpr bool two_byte = MODE == EPI_BF16 || MODE == EPI_BF16_BIAS;
+  constexpr int slab_cols = two_byte ? 64 : 32;
   const int grow0 = row0 + q * 32;
   const bool rows_in = grow0 < p.out_rows;
   // row scatter: this warp's 32 rows belong to one owner, whose buffer has its own tensor map
@@ -335,6 +369,8 @@ __device__ __forceinline__ void gemm_epilogue_tile_tma(const GemmParams &p, uint
   const CUtensorMap *tmap = p.tma_peer == 1 ? &p.tmPeer[owner] : &p.tmC;
   const int store_row = p.tma_peer == 1 ? grow0 - owner * p.peer_rows : grow0;
   const int store_plane = p.tma_peer == 1 ? p.peer_plane * p.splits + split : split;
+  uint8_t *const row_dst = stg + lane * 128;
+  const uint32_t swz = uint32_t(lane & 7) << 4;
   for (int c0 = 0; c0 < p.BN; c0 += slab_cols) {
     const int col0 = nn0 + c0;
     if (col0 >= p.out_cols) break;
@@ -353,81 +389,57 @@ __device__ __forceinline__ void gemm_epilogue_tile_tma(const GemmParams &p, uint
         tmem_ld_x32(t_addr + c0 + 32, hi);
       }
     }
+    EpiColumns next;
+    if ((MODE == EPI_BF16_BIAS || MODE == EPI_DEQUANT) && c0 + slab_cols < p.BN) next = epilogue_columns(p, col0 + slab_cols, lane);
     // the slab filled two stores ago must have been read by the copy engine before it is overwritten
     if (lane == 0) tma_store_wait_read<1>();
-    uint32_t bias2 = 0;   // bias of columns col0 + 2 lane, + 1 (bf16 pair), handed round by shuffles
-    if (two_byte && p.bias_kind == BIAS_BF16) {
-      const int c = col0 + 2 * lane;
-      const uint16_t *b = reinterpret_cast<const uint16_t *>(p.bias);
-      const uint32_t b0 = c < p.out_cols ? b[c] : 0u, b1 = c + 1 < p.out_cols ? b[c + 1] : 0u;
-      bias2 = b0 | (b1 << 16);
-    }
-    // int8 dequantisation: this lane holds scale / bias / compensation of column col0 + lane
-    float q_scale = 1.f, q_bias = 0.f;
-    int32_t q_comp = 0;
-    if (p.out_kind == OUT_DEQUANT_F32) {
-      const int c = col0 + lane;
-      if (c < p.out_cols) {
-        q_scale = p.scale[c];
-        if (p.bias_kind == BIAS_F32) q_bias = reinterpret_cast<const float *>(p.bias)[c];
-        if (p.comp) q_comp = p.comp[c];
-      }
-    }
     tmem_wait_ld();
     __syncwarp();
-    uint8_t *slab = stg + buf * 4096u;
-    if (p.out_kind == OUT_DEQUANT_F32) {
+    uint8_t *slab = row_dst + buf * 4096u;
+    if (two_byte) {
+      uint32_t y[32], nan[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = 4 * c + e;
-          const float sc = __shfl_sync(0xFFFFFFFFu, q_scale, j), bi = __shfl_sync(0xFFFFFFFFu, q_bias, j);
-          const int32_t cp = __shfl_sync(0xFFFFFFFFu, q_comp, j);
-          float f = __fmul_rn(float(int32_t(v[j]) - cp), sc);
-          if (p.bias_kind == BIAS_F32) f = __fadd_rn(f, bi);
-          if (p.relu) f = (f != f) ? f : (f > 0.f ? f : 0.f);
-          w[e] = __float_as_uint(f);
-        }
-        *reinterpret_cast<uint4 *>(slab + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+      for (int j = 0; j < 32; ++j) {
+        y[j] = pack_bf16x2_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));   // first rounding
+        if (MODE == EPI_BF16_BIAS) y[j] = bf16x2_add(y[j], __shfl_sync(0xFFFFFFFFu, cols.bias, j));   // second rounding
+        if (RELU) y[j] = bf16x2_relu(y[j]);
+        nan[j & 3] = bf16x2_max_nan(nan[j & 3], y[j]);
       }
-    } else if (two_byte) {
+      if ((bf16x2_nan_bits(nan[0]) | bf16x2_nan_bits(nan[1]) | bf16x2_nan_bits(nan[2]) | bf16x2_nan_bits(nan[3])) & 0x80008000u) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = 4 * c + e;   // pair index: columns 2j, 2j + 1 of the slab
-          uint32_t y = pack_bf16x2_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));   // first rounding
-          if (p.bias_kind == BIAS_BF16) {
-            const uint32_t bb = __shfl_sync(0xFFFFFFFFu, bias2, j);
-            const float f0 = __fadd_rn(__uint_as_float(y << 16), __uint_as_float(bb << 16));
-            const float f1 = __fadd_rn(__uint_as_float(y & 0xFFFF0000u), __uint_as_float(bb & 0xFFFF0000u));
-            y = pack_bf16x2_rn(f0, f1);                                                             // second rounding
-          }
-          if (p.relu) y = bf16x2_relu(y);
-          w[e] = bf16x2_fix_nan(y);
-        }
-        *reinterpret_cast<uint4 *>(slab + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int j = 0; j < 32; ++j) y[j] = bf16x2_fix_nan(y[j]);
       }
-    } else {
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<uint4 *>(slab + lane * 128 + ((c ^ (lane & 7)) << 4)) =
-            make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+        *reinterpret_cast<uint4 *>(slab + ((uint32_t(c) << 4) ^ swz)) = make_uint4(y[4 * c], y[4 * c + 1], y[4 * c + 2], y[4 * c + 3]);
+    } else {
+      if (MODE == EPI_DEQUANT) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const int32_t cp = int32_t(__shfl_sync(0xFFFFFFFFu, cols.comp, j));
+          float f = __fmul_rn(float(int32_t(v[j]) - cp), __uint_as_float(__shfl_sync(0xFFFFFFFFu, cols.scale, j)));
+          if (p.bias_kind == BIAS_F32) f = __fadd_rn(f, __uint_as_float(__shfl_sync(0xFFFFFFFFu, cols.bias, j)));
+          if (RELU) f = (f != f) ? f : (f > 0.f ? f : 0.f);
+          v[j] = __float_as_uint(f);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<uint4 *>(slab + ((uint32_t(c) << 4) ^ swz)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
     }
     fence_proxy_async();   // generic-proxy writes of the slab -> visible to the copy engine
     __syncwarp();
     if (lane == 0 && rows_in) {
+      const uint32_t src = smem_u32(stg + buf * 4096u);
       if (p.tma_peer == 2) {
-        for (int d = 0; d < p.n_peers; ++d) tma_store_3d(&p.tmPeer[d], smem_u32(slab), col0, grow0, 0);
+        for (int d = 0; d < p.n_peers; ++d) tma_store_3d(&p.tmPeer[d], src, col0, grow0, 0);
       } else {
-        tma_store_3d(tmap, smem_u32(slab), col0, store_row, store_plane);
+        tma_store_3d(tmap, src, col0, store_row, store_plane);
       }
       tma_store_commit();
     }
     buf ^= 1u;
+    cols = next;
   }
   if (p.tma_peer == 1 && p.signal_peer[0] != nullptr) {
     // the warp's rows of this tile are on their way to their owner: once the copy engine has completed the stores
@@ -436,6 +448,31 @@ __device__ __forceinline__ void gemm_epilogue_tile_tma(const GemmParams &p, uint
     if (lane == 0 && rows_in) {
       tma_store_wait<0>();
       publish_and_count(p.signal_peer[owner]);
+    }
+  }
+}
+
+template <int KIND>
+__device__ __forceinline__ void gemm_epilogue_tile_tma(const GemmParams &p, uint32_t t_addr, int row0, int nn0, int split,
+                                                       int q, int lane, uint8_t *stg, uint32_t &buf,
+                                                       const EpiColumns &cols) {
+  const int mode = epilogue_mode(p);
+  if (KIND == 0) {
+    if (mode == EPI_BF16_BIAS) {
+      if (p.relu) epilogue_tile_tma<KIND, EPI_BF16_BIAS, true>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
+      else        epilogue_tile_tma<KIND, EPI_BF16_BIAS, false>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
+    } else if (mode == EPI_BF16) {
+      if (p.relu) epilogue_tile_tma<KIND, EPI_BF16, true>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
+      else        epilogue_tile_tma<KIND, EPI_BF16, false>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
+    } else {
+      epilogue_tile_tma<KIND, EPI_RAW, false>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
+    }
+  } else {
+    if (mode == EPI_DEQUANT) {
+      if (p.relu) epilogue_tile_tma<KIND, EPI_DEQUANT, true>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
+      else        epilogue_tile_tma<KIND, EPI_DEQUANT, false>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
+    } else {
+      epilogue_tile_tma<KIND, EPI_RAW, false>(p, t_addr, row0, nn0, split, q, lane, stg, buf, cols);
     }
   }
 }

@@ -387,12 +387,23 @@ __device__ __forceinline__ uint32_t bf16x2_fix_nan(uint32_t w) {
   }
   return w;
 }
-// max(x, +0) on a packed pair, NaN propagating (arith.maximumf): the NaN comes back canonical and is
-// patched by bf16x2_fix_nan.
-__device__ __forceinline__ uint32_t bf16x2_relu(uint32_t w) {
+// Bits 15 / 31 of the result say that the low / high half of `w` is the NaN that cvt.rn and the packed bf16 arithmetic
+// return (0x7FFF); results of several words may be or-ed and tested once.
+__device__ __forceinline__ uint32_t bf16x2_nan_bits(uint32_t w) { return (w & 0x7FFF7FFFu) + 0x00010001u; }
+// a + b on packed pairs, each rounded once to nearest even: the same bits as adding in f32 and rounding that sum (the f32
+// sum of two bf16 values is inexact only when one is below 2^-15 of the other, and then both ways return the larger one).
+__device__ __forceinline__ uint32_t bf16x2_add(uint32_t a, uint32_t b) {
   uint32_t r;
-  asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0u));
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
+__device__ __forceinline__ uint32_t bf16x2_max_nan(uint32_t a, uint32_t b) {   // propagates NaN
+  uint32_t r;
+  asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// max(x, +0) on a packed pair, NaN propagating (arith.maximumf): the NaN comes back canonical and is
+// patched by bf16x2_fix_nan.
+__device__ __forceinline__ uint32_t bf16x2_relu(uint32_t w) { return bf16x2_max_nan(w, 0u); }
 
 } // namespace gcb
