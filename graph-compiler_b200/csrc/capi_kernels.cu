@@ -50,23 +50,17 @@ static void require(bool ok, const char *msg) {
   if (!ok) throw std::invalid_argument(msg);
 }
 
-// bf16 matmul: tensor-core path when TMA can address both operands, else the
-// exact-order SIMT kernel (same numerics, no alignment demands).
+// bf16 matmul of any operand layout (rows TMA cannot address are packed first).
 static void matmul_bf16_any(const void *A, const void *B, const void *bias, void *Y, int64_t M, int64_t N, int64_t K,
                             int ta, int tb, int relu, const MatmulConfig *force, cudaStream_t s) {
   require(A && B && Y, "null tensor pointer");
   require(M > 0 && N > 0 && K > 0, "matmul dimensions must be positive");
-  const bool ok = tma_compatible(A, ta ? M : K, 2) && tma_compatible(B, tb ? K : N, 2);
-  if (!ok) {
-    matmul_simt(A, B, bias, Y, M, N, K, ta, tb, 1, relu, s);
-    return;
-  }
   MatmulArgs a;
   a.A = A; a.B = B; a.M = M; a.N = N; a.K = K; a.trans_a = ta; a.trans_b = tb;
   a.out_kind = OUT_BF16; a.out = Y;
   a.bias_kind = bias ? BIAS_BF16 : BIAS_NONE; a.bias = bias; a.relu = relu;
   a.force = force;
-  matmul_tc(a, s);
+  matmul_bf16_any_layout(a, s);
 }
 
 } // namespace gcb
@@ -300,7 +294,7 @@ GCB_EXPORT int gcb200_matmul_f32(const float *A, const float *B, const float *bi
                                  int64_t K, int transpose_a, int transpose_b, int relu, void *stream) {
   return guarded([&] {
     require(A && B && Y && M > 0 && N > 0 && K > 0, "bad arguments");
-    matmul_simt(A, B, bias, Y, M, N, K, transpose_a, transpose_b, 0, relu, static_cast<cudaStream_t>(stream));
+    matmul_f32(A, B, bias, Y, M, N, K, transpose_a, transpose_b, relu, static_cast<cudaStream_t>(stream));
   });
 }
 

@@ -282,6 +282,7 @@ struct dnnl_graph_compiler_executable {
   static constexpr int kCanary = 0xA5;
   mutable DeviceBuffer splitk;          // split-K partial planes of this executable's matmul steps (they run one after
                                         // another on one stream, so one block sized for the largest request serves all)
+  mutable DeviceBuffer pack;            // likewise: packed copies of operands whose rows are no whole number of 16 bytes
 
   explicit dnnl_graph_compiler_executable(const std::string &json) : plan(build_plan(read_partition(json))) {}
   ~dnnl_graph_compiler_executable() {
@@ -330,6 +331,14 @@ struct dnnl_graph_compiler_executable {
           need = std::max(need, matmul_scratch_bytes(st.M / kRowChunks, st.N, st.K, 2, 2, d.sm_count));
       }
       if (need) splitk.reserve(need);
+      size_t packed = 0;
+      for (const Step &st : plan.steps) {
+        if (st.kind != StepKind::MATMUL || plan.part.tensors.at(st.in[0]).dtype != DType::BF16) continue;
+        MatmulArgs m;   // aligned bases: what the pitches alone ask for
+        m.M = st.M; m.N = st.N; m.K = st.K; m.trans_a = st.trans_a; m.trans_b = st.trans_b;
+        packed = std::max(packed, matmul_pack_bytes(m));
+      }
+      if (packed) pack.reserve(packed);
     }
     ready = true;
   }
@@ -411,15 +420,15 @@ struct dnnl_graph_compiler_executable {
       if (st.kind == StepKind::MATMUL || st.kind == StepKind::QMATMUL) {
         const bool q = st.kind == StepKind::QMATMUL;
         const bool bf16 = q || plan.part.tensors.at(st.in[0]).dtype == DType::BF16;
-        const bool tma = ((st.trans_a ? st.M : st.K) * (q ? 1 : 2)) % 16 == 0 && ((st.trans_b ? st.K : st.N) * (q ? 1 : 2)) % 16 == 0;
-        if (!bf16 || !tma) {
-          os << "matmul_simt_kernel (exact-order f32) " << st.M << "x" << st.N << "x" << st.K << "\n";
+        if (!bf16) {
+          os << "matmul_f32_kernel (exact-order f32) " << st.M << "x" << st.N << "x" << st.K << "\n";
           continue;
         }
+        const bool tma = (st.trans_a ? st.M : st.K) % 8 == 0 && (st.trans_b ? st.K : st.N) % 8 == 0;
         const MatmulConfig c = select_matmul_config(st.M, st.N, st.K, q ? 1 : 2, q ? 4 : 2, sm_count);
         os << "gemm_kernel<" << (q ? "u8 x s8" : "bf16") << (c.swapped ? ", weights on the MMA M side" : "") << "> " << st.M << "x" << st.N
            << "x" << st.K << " tile 128x" << c.bn << " splits " << c.splits << " stages " << c.stages << " K blocks/stage "
-           << std::max(1, c.kpb) << " grid " << c.grid << (c.splits > 1 ? " + reduce_planes" : "") << (q ? " + colsum_s8" : "") << "\n";
+           << std::max(1, c.kpb) << " grid " << c.grid << (!q && !tma ? " + pack_rows" : "") << (c.splits > 1 ? " + reduce_planes" : "") << (q ? " + colsum_s8" : "") << "\n";
       } else if (st.kind == StepKind::SDPA) {
         os << "attention_kernel B*H=" << st.batch * st.heads << " S=" << st.seq << " D=" << st.dim << " causal=" << st.causal << "\n";
       } else {
@@ -674,19 +683,18 @@ struct dnnl_graph_compiler_executable {
       const void *bias = st.has_bias ? addr(st.in[2]) : nullptr;
       if (A.dtype == DType::BF16) {
         const void *a = addr(st.in[0]), *b = addr(st.in[1]);
-        if (tma_compatible(a, st.trans_a ? st.M : st.K, 2) && tma_compatible(b, st.trans_b ? st.K : st.N, 2)) {
-          MatmulArgs m;
-          m.A = a; m.B = b; m.M = st.M; m.N = st.N; m.K = st.K; m.trans_a = st.trans_a; m.trans_b = st.trans_b;
-          m.out_kind = OUT_BF16; m.out = addr(st.out[0]);
-          m.bias_kind = bias ? BIAS_BF16 : BIAS_NONE; m.bias = bias; m.relu = st.relu;
-          m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;
-          matmul_tc(m, s);
-        } else {
-          matmul_simt(a, b, bias, addr(st.out[0]), st.M, st.N, st.K, st.trans_a, st.trans_b, 1, st.relu, s);
-        }
+        MatmulArgs m;
+        m.A = a; m.B = b; m.M = st.M; m.N = st.N; m.K = st.K; m.trans_a = st.trans_a; m.trans_b = st.trans_b;
+        m.out_kind = OUT_BF16; m.out = addr(st.out[0]);
+        m.bias_kind = bias ? BIAS_BF16 : BIAS_NONE; m.bias = bias; m.relu = st.relu;
+        m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;
+        const size_t need = matmul_pack_bytes(m);
+        if (need && need <= pack.bytes) matmul_bf16_packed(m, pack.ptr, s);
+        else matmul_bf16_any_layout(m, s);
       } else {
-        matmul_simt(addr(st.in[0]), addr(st.in[1]), bias, addr(st.out[0]), st.M, st.N, st.K, st.trans_a, st.trans_b, 0,
-                    st.relu, s);
+        matmul_f32(static_cast<const float *>(addr(st.in[0])), static_cast<const float *>(addr(st.in[1])),
+                   static_cast<const float *>(bias), static_cast<float *>(addr(st.out[0])), st.M, st.N, st.K, st.trans_a, st.trans_b,
+                   st.relu, s);
       }
       break;
     }

@@ -355,6 +355,35 @@ __device__ __forceinline__ EpiColumns epilogue_columns(const GemmParams &p, int 
   return e;
 }
 
+// Stores one staged slab of 32 rows from the warp's buffer, a row per step, for outputs whose base or pitch is no whole
+// number of 16 bytes: the lanes write consecutive 4-byte words (128 bytes of a row per instruction).  bf16 rows that start
+// half a word off are shifted by one element between neighbouring lanes.  nval: columns of the slab inside tile and output.
+template <bool TWO_BYTE>
+__device__ __forceinline__ void store_slab_rows(const GemmParams &p, const uint8_t *slab, int grow0, int col0, int nval, size_t plane, int lane) {
+  const int rows = min(32, p.out_rows - grow0);
+  uint8_t *g = reinterpret_cast<uint8_t *>(p.out) + (plane + size_t(grow0) * size_t(p.ld_out) + size_t(col0)) * (TWO_BYTE ? 2 : 4);
+  const size_t pitch = size_t(p.ld_out) * (TWO_BYTE ? 2 : 4);
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r, g += pitch) {
+    const uint32_t w = *reinterpret_cast<const uint32_t *>(slab + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+    if (!TWO_BYTE) {
+      if (lane < nval) reinterpret_cast<uint32_t *>(g)[lane] = w;
+      continue;
+    }
+    uint16_t *e = reinterpret_cast<uint16_t *>(g);
+    const uint32_t up = __shfl_down_sync(0xFFFFFFFFu, w, 1);
+    const int c = 2 * lane;   // this lane's columns: c, c + 1
+    if ((reinterpret_cast<uintptr_t>(g) & 2) == 0) {
+      if (c + 1 < nval) *reinterpret_cast<uint32_t *>(e + c) = w;
+      else if (c < nval) e[c] = uint16_t(w);
+    } else {
+      if (lane == 0 && nval > 0) e[0] = uint16_t(w);
+      if (lane < 31 && c + 2 < nval) *reinterpret_cast<uint32_t *>(e + c + 1) = (w >> 16) | (up << 16);
+      else if (c + 1 < nval) e[c + 1] = uint16_t(w >> 16);
+    }
+  }
+}
+
 // stg: this warp's two 4 KiB slabs (1 KiB aligned); buf: slab to fill next (kept by the caller across tiles).
 template <int KIND, int MODE, bool RELU>
 __device__ __forceinline__ void epilogue_tile_tma(const GemmParams &p, uint32_t t_addr, int row0, int nn0, int split,
@@ -374,7 +403,7 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams &p, uint32_t 
   for (int c0 = 0; c0 < p.BN; c0 += slab_cols) {
     const int col0 = nn0 + c0;
     if (col0 >= p.out_cols) break;
-    if (p.tma_peer != 1 && p.BN - c0 < slab_cols) {
+    if (p.tma_store && p.tma_peer != 1 && p.BN - c0 < slab_cols) {
       // the tile is not a whole number of slabs wide (BN a multiple of 16 only): the last 16, 32 or 48 columns
       // go from registers straight to global memory, 16 columns (32 or 64 contiguous bytes per row) at a time
       gemm_epilogue_tail<KIND>(p, t_addr, c0, col0, grow0 + lane, split, lane);
@@ -392,7 +421,7 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams &p, uint32_t 
     EpiColumns next;
     if ((MODE == EPI_BF16_BIAS || MODE == EPI_DEQUANT) && c0 + slab_cols < p.BN) next = epilogue_columns(p, col0 + slab_cols, lane);
     // the slab filled two stores ago must have been read by the copy engine before it is overwritten
-    if (lane == 0) tma_store_wait_read<1>();
+    if (p.tma_store && lane == 0) tma_store_wait_read<1>();
     tmem_wait_ld();
     __syncwarp();
     uint8_t *slab = row_dst + buf * 4096u;
@@ -426,6 +455,15 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams &p, uint32_t 
 #pragma unroll
       for (int c = 0; c < 8; ++c)
         *reinterpret_cast<uint4 *>(slab + ((uint32_t(c) << 4) ^ swz)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    }
+    if (!p.tma_store) {
+      __syncwarp();
+      const size_t plane = (p.splits > 1) ? size_t(split) * size_t(p.split_stride) : 0;
+      store_slab_rows<two_byte>(p, stg + buf * 4096u, grow0, col0, min(min(slab_cols, p.BN - c0), p.out_cols - col0), plane, lane);
+      __syncwarp();
+      buf ^= 1u;
+      cols = next;
+      continue;
     }
     fence_proxy_async();   // generic-proxy writes of the slab -> visible to the copy engine
     __syncwarp();

@@ -255,7 +255,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       tile_coords(p, tile, tm, tn);
       const uint32_t acc = tcount & 1u, acc_ph = (tcount >> 1) & 1u;
       EpiColumns cols;
-      if (!SWAPPED && p.tma_store) cols = epilogue_columns(p, tn * p.BN, lane);
+      if (!SWAPPED && (p.tma_store || p.row_store)) cols = epilogue_columns(p, tn * p.BN, lane);
       if (!mbar_wait(smem_u32(&bars->tmem_full[acc]), acc_ph)) {
         if (lane == 0) atomicExch(p.error, ERR_WAIT_TMEM_FULL);
         dead = true;
@@ -265,7 +265,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const uint32_t t_addr = tmem_base + acc * uint32_t(p.BN) + (uint32_t(q * 32) << 16);
       const int nn0 = tn * p.BN;                 // first MMA column of the tile
 
-      if (!SWAPPED && p.tma_store) gemm_epilogue_tile_tma<KIND>(p, t_addr, tm * kBM, nn0, split, q, lane, stg, slab, cols);
+      if (!SWAPPED && (p.tma_store || p.row_store)) gemm_epilogue_tile_tma<KIND>(p, t_addr, tm * kBM, nn0, split, q, lane, stg, slab, cols);
       else gemm_epilogue_tile<KIND, SWAPPED>(p, t_addr, tm * kBM, nn0, split, q, lane, stg);
       tc_fence_before();
       __syncwarp();

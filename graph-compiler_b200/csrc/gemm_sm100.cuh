@@ -86,6 +86,7 @@ struct GemmParams {
   // [planes][rows][cols] with a box of {128 bytes of columns, 32 rows, 1}; each epilogue warp hands its
   // 32 x 128-byte slabs to the copy engine instead of storing them itself.
   int tma_store;
+  int row_store;        // the same epilogue with the slabs stored row by row (outputs the copy engine cannot address)
   CUtensorMap tmC;
   // Row scatter through the copy engine (tma_peer = 1, with tma_store): tmPeer[d] covers owner d's receive buffer as
   // [planes][rows per peer][cols] f32 with the same box; a warp's 32-row slab goes to its owner's buffer with one

@@ -297,33 +297,35 @@ OperandGeom operand_geom(bool mn_major, int tile_mn, int elem_bytes, int kpb) {
 }
 
 CUtensorMap operand_tmap(OperandGeom &g, ElemType t, int elem_bytes, const void *ptr, int64_t mn_total,
-                                int64_t k_total, int tile_mn, int kpb) {
+                                int64_t k_total, int tile_mn, int kpb, int64_t ld) {
   const uint32_t bk = 128 / elem_bytes;
-  if (g.mn_major && elem_bytes == 2 && mn_total % int64_t(g.box_mn) == 0 && tile_mn % int(g.box_mn) == 0) {
+  if (!ld) ld = g.mn_major ? mn_total : k_total;   // elements from one row in memory to the next
+  if (g.mn_major && elem_bytes == 2 && ld % int64_t(g.box_mn) == 0 && tile_mn % int(g.box_mn) == 0) {
     // memory [k_total][mn_total] seen as [group][k][128 bytes]: one copy brings all 64-wide (128-byte)
     // groups of the tile, landing as consecutive [rows x 128 B] blocks — the layout the MMA reads.
-    // Only when MN is a whole number of groups: a partial last group would make the copy read past
+    // Only when the pitch is a whole number of groups: a partial last group would make the copy read past
     // the end of the last row; and only when the tile is a whole number of groups wide, so that every
     // tile starts on a group boundary (tiles of 16 x odd columns take one 2-D copy per group instead).  16-bit operands only: the same 3-D form on 8-bit operands returned
     // wrong data for the second group at small N on B200, so those keep one 2-D copy per group.
     g.one_load = 1;
-    return make_tmap_3d(t, ptr, g.box_mn, uint64_t(k_total), uint64_t(mn_total) / g.box_mn,
-                        uint64_t(mn_total) * elem_bytes, 128, g.box_mn, bk * uint32_t(kpb), g.boxes);
+    return make_tmap_3d(t, ptr, g.box_mn, uint64_t(k_total), uint64_t(ceil_div(mn_total, g.box_mn)),
+                        uint64_t(ld) * elem_bytes, 128, g.box_mn, bk * uint32_t(kpb), g.boxes);
   }
   if (!g.mn_major) {  // memory [mn_total][k_total], K contiguous
-    if (kpb > 1 && elem_bytes == 2 && k_total % int64_t(bk) == 0) {
+    if (kpb > 1 && elem_bytes == 2 && ld % int64_t(bk) == 0) {
       // [K block][mn][128 bytes]: one copy brings the stage's K blocks as consecutive swizzled tiles.
-      // Only when K is a whole number of blocks (a partial block would read into the next row).
+      // Only when the pitch is a whole number of blocks (a partial block would read into the next row; the padding of a
+      // packed operand is zero).
       g.one_load = 1;
       g.k3d = 1;
-      return make_tmap_3d(t, ptr, bk, uint64_t(mn_total), uint64_t(k_total) / bk, uint64_t(k_total) * elem_bytes, 128, bk,
+      return make_tmap_3d(t, ptr, bk, uint64_t(mn_total), uint64_t(ceil_div(k_total, bk)), uint64_t(ld) * elem_bytes, 128, bk,
                           uint32_t(tile_mn), uint32_t(kpb));
     }
-    return make_tmap_2d(t, ptr, uint64_t(k_total), uint64_t(mn_total), uint64_t(k_total) * elem_bytes, bk,
+    return make_tmap_2d(t, ptr, uint64_t(k_total), uint64_t(mn_total), uint64_t(ld) * elem_bytes, bk,
                         uint32_t(tile_mn));
   }
   // memory [k_total][mn_total], MN contiguous
-  return make_tmap_2d(t, ptr, uint64_t(mn_total), uint64_t(k_total), uint64_t(mn_total) * elem_bytes, g.box_mn,
+  return make_tmap_2d(t, ptr, uint64_t(mn_total), uint64_t(k_total), uint64_t(ld) * elem_bytes, g.box_mn,
                       bk * uint32_t(kpb));
 }
 
@@ -352,17 +354,17 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   // operand roles in MMA orientation
   const void *pa, *pb;
   bool a_mn, b_mn;
-  int64_t mn_a, mn_b;
+  int64_t mn_a, mn_b, ld_a, ld_b;
   ElemType ta, tb;
   uint32_t fa, fb;
   if (!cfg.swapped) {
-    pa = a.A; a_mn = a.trans_a != 0; mn_a = a.M;
-    pb = a.B; b_mn = a.trans_b == 0; mn_b = a.N;
+    pa = a.A; a_mn = a.trans_a != 0; mn_a = a.M; ld_a = a.lda;
+    pb = a.B; b_mn = a.trans_b == 0; mn_b = a.N; ld_b = a.ldb;
     ta = a.int8 ? ElemType::U8 : ElemType::BF16; tb = a.int8 ? ElemType::S8 : ElemType::BF16;
     fa = a.int8 ? 0u : 1u; fb = 1u;
   } else {
-    pa = a.B; a_mn = a.trans_b == 0; mn_a = a.N;
-    pb = a.A; b_mn = a.trans_a != 0; mn_b = a.M;
+    pa = a.B; a_mn = a.trans_b == 0; mn_a = a.N; ld_a = a.ldb;
+    pb = a.A; b_mn = a.trans_a != 0; mn_b = a.M; ld_b = a.lda;
     ta = a.int8 ? ElemType::S8 : ElemType::BF16; tb = a.int8 ? ElemType::U8 : ElemType::BF16;
     fa = 1u; fb = a.int8 ? 0u : 1u;
   }
@@ -389,8 +391,8 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   while (cols < uint32_t(2 * p.BN)) cols <<= 1;
   p.tmem_cols = cols;
 
-  const CUtensorMap tmA = operand_tmap(p.a, ta, eb, pa, mn_a, a.K, 128, kpb);
-  const CUtensorMap tmB = operand_tmap(p.b, tb, eb, pb, mn_b, a.K, pair ? p.BN / 2 : p.BN, kpb);
+  const CUtensorMap tmA = operand_tmap(p.a, ta, eb, pa, mn_a, a.K, 128, kpb, ld_a);
+  const CUtensorMap tmB = operand_tmap(p.b, tb, eb, pb, mn_b, a.K, pair ? p.BN / 2 : p.BN, kpb, ld_b);
 
   if (a.n_peers > 0) {
     // f32 partial planes ([planes][M][N], pitch N) or finished results (bf16 / dequantised f32 with their
@@ -471,6 +473,8 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
       p.tmC = make_tmap_3d(ct, p.out, uint64_t(a.N), uint64_t(a.M), uint64_t(std::max(1, p.splits)), uint64_t(p.ld_out) * esz,
                            split ? uint64_t(p.split_stride) * esz : uint64_t(a.M) * uint64_t(p.ld_out) * esz, 128 / esz, 32, 1);
       p.tma_store = 1;
+    } else if (plain) {
+      p.row_store = 1;
     }
   }
   // Row scatter of f32 partial sums: through the copy engine as well, one tensor map per owner (tile widths that are
@@ -736,83 +740,6 @@ void colsum_s8(const int8_t *W, int32_t *comp, int64_t K, int64_t N, int32_t zp,
   GCB_CUDA(cudaMemsetAsync(comp, 0, size_t(N) * 4, stream));
   dim3 grid(unsigned((N + 255) / 256), unsigned(std::min<int64_t>(K, 64)));
   colsum_s8_kernel<<<grid, 256, 0, stream>>>(W, comp, K, N, zp);
-  GCB_CUDA(cudaGetLastError());
-  count_launch();
-}
-
-// Exact-order SIMT matmul: every output element accumulates k ascending with a
-// separate multiply and add, the arithmetic of the reference's scalar loops
-// (BrgemmNaive.cpp:46-99).  64x64 output tile, 16-deep K slabs in shared memory.
-template <int IN_KIND>
-__global__ void __launch_bounds__(256) matmul_simt_kernel(const void *Ap, const void *Bp, const void *biasp, void *outp,
-                                                         int M, int N, int K, int ta, int tb, int relu) {
-  __shared__ float As[16][65];
-  __shared__ float Bs[16][65];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  auto ld = [&](const void *base, long long idx) -> float {
-    if (IN_KIND == 0) return reinterpret_cast<const float *>(base)[idx];
-    return bf16_bits_to_f32(reinterpret_cast<const uint16_t *>(base)[idx]);
-  };
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-      const int kk = e / 64, mm = e % 64;
-      const int k = k0 + kk;
-      float av = 0.f, bv = 0.f;
-      if (k < K && m0 + mm < M) av = ta ? ld(Ap, (long long)k * M + (m0 + mm)) : ld(Ap, (long long)(m0 + mm) * K + k);
-      if (k < K && n0 + mm < N) bv = tb ? ld(Bp, (long long)(n0 + mm) * K + k) : ld(Bp, (long long)k * N + (n0 + mm));
-      As[kk][mm] = av;
-      Bs[kk][mm] = bv;
-    }
-    __syncthreads();
-    const int klim = min(16, K - k0);
-    for (int kk = 0; kk < klim; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(a[i], b[j]));
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-      if (m >= M || n >= N) continue;
-      if (IN_KIND == 0) {
-        float v = acc[i][j];
-        if (biasp) v = __fadd_rn(v, reinterpret_cast<const float *>(biasp)[n]);
-        if (relu) v = (v != v) ? v : (v > 0.f ? v : 0.f);
-        reinterpret_cast<float *>(outp)[(long long)m * N + n] = v;
-      } else {
-        uint32_t y = f32_to_bf16_bits(acc[i][j]);
-        if (biasp)
-          y = f32_to_bf16_bits(__fadd_rn(bf16_bits_to_f32(y), bf16_bits_to_f32(reinterpret_cast<const uint16_t *>(biasp)[n])));
-        if (relu) { const float f = bf16_bits_to_f32(y); y = (f != f) ? y : (f > 0.f ? y : 0u); }
-        reinterpret_cast<uint16_t *>(outp)[(long long)m * N + n] = uint16_t(y);
-      }
-    }
-}
-
-void matmul_simt(const void *A, const void *B, const void *bias, void *out, int64_t M, int64_t N, int64_t K,
-                 int trans_a, int trans_b, int in_kind, int relu, cudaStream_t stream) {
-  device_state();
-  dim3 grid(unsigned((N + 63) / 64), unsigned((M + 63) / 64));
-  if (in_kind == 0)
-    matmul_simt_kernel<0><<<grid, 256, 0, stream>>>(A, B, bias, out, int(M), int(N), int(K), trans_a, trans_b, relu);
-  else
-    matmul_simt_kernel<1><<<grid, 256, 0, stream>>>(A, B, bias, out, int(M), int(N), int(K), trans_a, trans_b, relu);
   GCB_CUDA(cudaGetLastError());
   count_launch();
 }

@@ -78,8 +78,9 @@ bool tma_compatible(const void *ptr, int64_t row_elems, int elem_bytes);
 // M or N side; K contiguous in memory unless mn_major).
 OperandGeom operand_geom(bool mn_major, int tile_mn, int elem_bytes, int kpb = 1);
 // (sets g.one_load when the operand can be fetched with a single 3-D copy per stage)
+// ld: pitch in elements (0: dense)
 CUtensorMap operand_tmap(OperandGeom &g, ElemType t, int elem_bytes, const void *ptr, int64_t mn_total,
-                         int64_t k_total, int tile_mn, int kpb = 1);
+                         int64_t k_total, int tile_mn, int kpb = 1, int64_t ld = 0);
 CUtensorMap make_tmap_3d(ElemType t, const void *ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
                          uint64_t stride2_bytes, uint32_t b0, uint32_t b1, uint32_t b2);
 
@@ -92,6 +93,7 @@ struct MatmulArgs {
   int int8 = 0;                 // 0: bf16 x bf16 -> f32;  1: u8 x s8 -> s32
   int out_kind = OUT_BF16;
   void *out = nullptr;
+  int64_t lda = 0, ldb = 0;     // operand pitch in elements where it is larger than the row (0: dense)
   int64_t ld_out = 0;           // 0 -> N
   int bias_kind = BIAS_NONE;
   const void *bias = nullptr;
@@ -128,10 +130,17 @@ void reduce_planes(const void *parts, int nparts, int64_t plane, void *out, int6
 // comp[n] = zp * sum_k W[k,n]   (W s8 [K,N] row-major)
 void colsum_s8(const int8_t *W, int32_t *comp, int64_t K, int64_t N, int32_t zp, cudaStream_t stream);
 
-// Exact-order f32 SIMT matmul (k ascending, separate multiply and add) for f32
-// graphs and for operand layouts TMA cannot address.  in_kind: 0 f32, 1 bf16.
-void matmul_simt(const void *A, const void *B, const void *bias, void *out, int64_t M, int64_t N, int64_t K,
-                 int trans_a, int trans_b, int in_kind, int relu, cudaStream_t stream);
+// Exact-order f32 matmul (k ascending, separate multiply and add) for f32 graphs (matmul_f32.cu).
+void matmul_f32(const float *A, const float *B, const float *bias, float *out, int64_t M, int64_t N, int64_t K, int trans_a,
+                int trans_b, int relu, cudaStream_t stream);
+
+// bf16 matmul whose operand rows the copy engine cannot address (base or pitch not a whole number of 16 bytes): such
+// operands are first copied into `pack`, rows padded to whole 128-byte groups with zeros, and the tensor-core kernels run
+// on the copies.  pack_bytes: what a call needs (0: both operands can be used as they are).
+size_t matmul_pack_bytes(const MatmulArgs &a);
+void matmul_bf16_packed(const MatmulArgs &a, void *pack, cudaStream_t stream);
+// The same with the copies in stream-ordered memory of this library's own pool (direct launchers: any stream, any thread).
+void matmul_bf16_any_layout(const MatmulArgs &a, cudaStream_t stream);
 
 int read_device_error(cudaStream_t stream); // synchronises the stream; returns and clears the error word
 
