@@ -47,7 +47,7 @@ def test_bf16_layouts_without_alignment(M, N, K, ta, tb, bias, relu, skip):
 @pytest.mark.parametrize("M,N,K,ta,tb", [(700, 1300, 40, 0, 0), (65, 66, 17, 1, 0), (40, 130, 33, 0, 1), (5, 768, 100, 0, 0), (17, 31, 16, 1, 1),
                                          (640, 1024, 16, 1, 1), (1, 1, 1, 0, 0)])
 def test_f32_bits(M, N, K, ta, tb):
-    """64 x 64, 32 x 32 and 16 x 32 tiles, whole and ragged, K slabs whole and cut: the oracle's bits."""
+    """64 x 64, 32 x 32 and 16 x 16 tiles, whole and ragged, K slabs whole and cut: the oracle's bits."""
     A, B, b = (_rand(s, i).float().numpy() for i, s in enumerate([(M, K), (K, N), (N,)]))
     dev = lambda x, t: torch.from_numpy(np.ascontiguousarray(x.T if t else x)).to(DEV)
     Y = lib.matmul_f32(dev(A, ta), dev(B, tb), dev(b, 0), True, bool(ta), bool(tb))
