@@ -1,11 +1,12 @@
-"""Build libGcDnnlApi.so (sm_100a) in-tree.
+"""Build libGcDnnlApi.so (sm_100a) and its Python call path in-tree.
 
     python graph-compiler_b200/build.py [--force] [--verbose]
 
 Every .cu/.cpp under csrc/ is compiled to an object with
 ``nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo`` (objects are rebuilt
 only when a source or header is newer) and linked into
-``graph-compiler_b200/lib/libGcDnnlApi.so``.  nvcc cross-compiles, so this works
+``graph-compiler_b200/lib/libGcDnnlApi.so``; binding/gcb200_host.cpp (plain CPython API) becomes
+``lib/_gcb200_host.so``.  nvcc cross-compiles, so this works
 on a machine without a GPU.
 """
 from __future__ import annotations
@@ -16,12 +17,14 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libGcDnnlApi.so")
+HOST = os.path.join(LIBDIR, "_gcb200_host.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -69,6 +72,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
         os.replace(tmp, LIB)
+    src = os.path.join(HERE, "binding", "gcb200_host.cpp")
+    if force or not os.path.exists(HOST) or os.path.getmtime(HOST) < max(os.path.getmtime(src), hdr):
+        tmp = HOST + ".tmp"
+        cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], src,
+               "-o", tmp, "-L", LIBDIR, "-lGcDnnlApi", "-Wl,-rpath,$ORIGIN"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("the Python binding did not build")
+        os.replace(tmp, HOST)
     return LIB
 
 

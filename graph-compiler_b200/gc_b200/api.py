@@ -130,6 +130,11 @@ class Executable:
 
     def execute(self, inputs: Dict[int, object], outputs: Dict[int, object]) -> None:
         """Synchronous, like the reference: results are in ``outputs`` on return."""
+        st = (_lib._host or _lib.host()).execute(self._h.value if self._h else 0, inputs, outputs, None)
+        if st == SUCCESS:
+            return
+        if st is not None:
+            raise DnnlError(st, _lib.load().gcb200_last_error().decode(errors="replace"))
         i_arr, k1 = _pack(inputs)
         o_arr, k2 = _pack(outputs)
         st = _bind().dnnl_graph_compiler_execute(self._h, i_arr, o_arr)
@@ -138,6 +143,11 @@ class Executable:
 
     def execute_on_stream(self, inputs, outputs, stream=None) -> None:
         """Device tensors only: enqueue on ``stream`` (default: torch's current) and return."""
+        st = (_lib._host or _lib.host()).execute(self._h.value if self._h else 0, inputs, outputs, stream.cuda_stream if stream else True)
+        if st == SUCCESS:
+            return
+        if st is not None:
+            raise DnnlError(st, _lib.load().gcb200_last_error().decode(errors="replace"))
         import torch
 
         s = C.c_void_p((stream or torch.cuda.current_stream()).cuda_stream)

@@ -8,9 +8,11 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(os.path.dirname(_HERE), "lib", "libGcDnnlApi.so")
+HOST_PATH = os.path.join(os.path.dirname(_HERE), "lib", "_gcb200_host.so")
 
 _i64, _u64, _i32, _int, _vp, _f32 = C.c_int64, C.c_uint64, C.c_int32, C.c_int, C.c_void_p, C.c_float
 
@@ -107,6 +109,34 @@ def load() -> C.CDLL:
     return lib
 
 
+_host = None         # the compiled module, once torch is there to be bound
+_host_module = None
+
+
+def host():
+    """The compiled call path of the small, repeated calls (binding/gcb200_host.cpp)."""
+    global _host, _host_module
+    if _host is not None:
+        return _host
+    if _host_module is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise FileNotFoundError(f"{HOST_PATH} is missing: build it with `python graph-compiler_b200/build.py`")
+        import importlib.machinery
+        import importlib.util
+
+        loader = importlib.machinery.ExtensionFileLoader("_gcb200_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_gcb200_host", loader))
+        loader.exec_module(mod)
+        mod.setup(type(None), None, None, None)
+        _host_module = mod
+    torch = sys.modules.get("torch")   # a program that holds tensors has imported it
+    if torch is not None:
+        _host_module.setup(torch.Tensor, torch.bfloat16, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream)
+        _host = _host_module
+    return _host_module
+
+
 def check(status: int) -> None:
     if status != 0:
         raise GcB200Error(status, load().gcb200_last_error().decode(errors="replace"))
@@ -119,7 +149,7 @@ def _ptr(t):
 def _stream():
     import torch
 
-    return _vp(torch.cuda.current_stream().cuda_stream)
+    return _vp(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def sm_count() -> int:
@@ -187,6 +217,11 @@ def tune_cache_clear():
 # ----------------------------------------------------------------------------- launchers on torch CUDA tensors
 def matmul_bf16(A, B, bias=None, relu=False, transpose_a=False, transpose_b=False, out=None, cfg: MatmulConfig | None = None):
     """Y = act(bf16(bf16(op(A).op(B)) + bias)) on bf16 CUDA tensors."""
+    if out is not None and cfg is None:
+        st = (_host or host()).matmul_bf16(A, B, bias, relu, transpose_a, transpose_b, out)
+        if st:
+            check(st)
+        return out
     import torch
 
     assert A.is_cuda and A.dtype == torch.bfloat16 and A.is_contiguous() and B.is_contiguous()
@@ -328,6 +363,11 @@ def matmul_f32(A, B, bias=None, relu=False, transpose_a=False, transpose_b=False
 
 def attention_bf16(Q, K, V, scale: float, causal: bool = False, out=None):
     """Fused attention on bf16 CUDA tensors [..., S, D] (leading dims are independent units)."""
+    if out is not None:
+        st = (_host or host()).attention_bf16(Q, K, V, scale, causal, out)
+        if st:
+            check(st)
+        return out
     import torch
 
     assert Q.is_contiguous() and K.is_contiguous() and V.is_contiguous() and Q.dtype == torch.bfloat16
