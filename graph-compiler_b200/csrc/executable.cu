@@ -202,6 +202,29 @@ __global__ void __launch_bounds__(256) reduce_block_kernel(ReduceParams p, const
   }
 }
 
+// Brings a block of pinned host memory over the bus: the SMs read it in place.  Enough loads are in flight (16 bytes per
+// thread, up to 64 blocks of 256) for the bus rate at its latency; a copy engine has the same rate but starts later and
+// hands over to the next kernel through a semaphore.  Both ends are multiples of 16 bytes.
+__global__ void __launch_bounds__(256) fetch_pinned_kernel(uint4 *dst, const uint4 *src, int n) {
+  pdl_launch_dependents();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) dst[i] = __ldcs(src + i);
+  pdl_wait();   // what runs behind this kernel runs behind everything ahead of it
+}
+static void fetch_pinned(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  const int n = int(bytes / 16);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(std::min(64, (n + 255) / 256)));
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  GCB_CUDA(cudaLaunchKernelEx(&cfg, fetch_pinned_kernel, static_cast<uint4 *>(dst), static_cast<const uint4 *>(src), n));
+  count_launch();
+}
+
 static int ew_dtype(DType t) {
   switch (t) {
   case DType::F32: return 0;
@@ -265,7 +288,6 @@ struct dnnl_graph_compiler_executable {
   mutable cudaStream_t stream = nullptr;
   mutable cudaStream_t copy_in = nullptr, copy_out = nullptr;   // host copies that overlap the first / last matmul
   mutable cudaEvent_t ev_in[4] = {}, ev_out[4] = {};
-  mutable int *host_code = nullptr;                             // pinned: the device error word after a call
   // Replay of the launch list as a CUDA graph when a call repeats an earlier call's device addresses:
   // the first call runs eagerly (it also sizes the workspaces), the second is captured, later ones replay.
   struct GraphEntry {
@@ -278,13 +300,44 @@ struct dnnl_graph_compiler_executable {
   mutable unsigned long long graph_clock = 0;
   mutable DeviceBuffer arena;
   mutable std::vector<DeviceBuffer> in_stage, out_stage;
+  // Small pageable host tensors of the synchronous call: one pinned block for the inputs, brought over by a kernel that
+  // reads it (no copy engine, no driver staging), and one for the results, which the last kernels write directly.
+  struct PinnedBlock {
+    uint8_t *ptr = nullptr;
+    size_t bytes = 0;
+    void reserve(size_t n) {
+      if (n <= bytes) return;
+      if (ptr) cudaFreeHost(ptr);
+      ptr = nullptr;
+      bytes = 0;
+      GCB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&ptr), n, cudaHostAllocMapped));
+      bytes = n;
+    }
+    ~PinnedBlock() {
+      if (ptr) cudaFreeHost(ptr);
+    }
+  };
+  mutable PinnedBlock small_in_host, small_out_host;
+  mutable DeviceBuffer small_in;
   mutable std::vector<char> comp_ready; // per QMATMUL scratch: column sums computed for a cached constant weight
   static constexpr int kCanary = 0xA5;
   mutable DeviceBuffer splitk;          // split-K partial planes of this executable's matmul steps (they run one after
                                         // another on one stream, so one block sized for the largest request serves all)
   mutable DeviceBuffer pack;            // likewise: packed copies of operands whose rows are no whole number of 16 bytes
 
-  explicit dnnl_graph_compiler_executable(const std::string &json) : plan(build_plan(read_partition(json))) {}
+  std::vector<char> host_writable;      // per output: its step may write it in host memory (nothing reads it back, and
+                                        // the step is a kernel with plain stores)
+  explicit dnnl_graph_compiler_executable(const std::string &json) : plan(build_plan(read_partition(json))) {
+    for (size_t id : plan.part.output_ids) {
+      bool ok = true;
+      for (const Step &st : plan.steps) {
+        ok &= std::find(st.in.begin(), st.in.end(), id) == st.in.end();
+        if (std::find(st.out.begin(), st.out.end(), id) != st.out.end())
+          ok &= st.kind != StepKind::COPY && !(st.kind == StepKind::QMATMUL && st.raw_acc);
+      }
+      host_writable.push_back(ok);
+    }
+  }
   ~dnnl_graph_compiler_executable() {
     if (stream) cudaStreamDestroy(stream);
     if (copy_in) cudaStreamDestroy(copy_in);
@@ -293,7 +346,6 @@ struct dnnl_graph_compiler_executable {
       if (ev_in[i]) cudaEventDestroy(ev_in[i]);
       if (ev_out[i]) cudaEventDestroy(ev_out[i]);
     }
-    if (host_code) cudaFreeHost(host_code);
     for (GraphEntry &g : graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
   }
@@ -309,7 +361,6 @@ struct dnnl_graph_compiler_executable {
       GCB_CUDA(cudaEventCreateWithFlags(&ev_in[i], cudaEventDisableTiming));
       GCB_CUDA(cudaEventCreateWithFlags(&ev_out[i], cudaEventDisableTiming));
     }
-    GCB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&host_code), sizeof(int), cudaHostAllocDefault));
     if (plan.arena_bytes) arena.reserve(plan.arena_bytes);
     if (plan.guard_bytes && plan.arena_bytes) GCB_CUDA(cudaMemset(arena.ptr, kCanary, plan.arena_bytes));
     gcLogD("executable prepared on device ", device, ": arena ", plan.arena_bytes, " bytes, ", plan.steps.size(), " steps, guard bands ",
@@ -350,15 +401,22 @@ struct dnnl_graph_compiler_executable {
     throw std::invalid_argument("Tensor not found");
   }
 
-  static bool on_device(const void *p) {
+  enum class Where { DEVICE, PINNED, PAGEABLE };
+  static Where where(const void *p) {
     cudaPointerAttributes at;
-    cudaError_t e = cudaPointerGetAttributes(&at, p);
-    if (e != cudaSuccess) {
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
       cudaGetLastError();
-      return false;
+      return Where::PAGEABLE;
     }
-    return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
+    return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged ? Where::DEVICE
+           : at.type == cudaMemoryTypeHost                                   ? Where::PINNED
+                                                                             : Where::PAGEABLE;
   }
+  // Up to these sizes the extra pass over pageable memory (10 to 20 GB/s on one core) is cheaper than the driver's staging
+  // copies, each of which costs 10 to 20 us beyond a pinned one whatever its size; above, the driver's pipelined copy is
+  // as fast.
+  static constexpr size_t kSmallIn = 1 << 20, kSmallOut = 256 << 10;
+  static size_t padded(size_t n) { return (n + 255) / 256 * 256; }
 
   void check_dims(const dnnl_graph_compiler_tensor *t, const LogicalTensor &lt) const {
     if (t->ndims > DNNL_MAX_NDIMS) throw std::invalid_argument("Number of dimensions > DNNL_MAX_NDIMS");
@@ -456,7 +514,15 @@ struct dnnl_graph_compiler_executable {
     cudaStream_t s = own_stream ? stream : user_stream;
     const Partition &p = plan.part;
     const size_t ni = p.input_ids.size(), no = p.output_ids.size();
-    std::vector<void *> in_ptr(ni), out_ptr(no), out_host(no, nullptr);
+    std::vector<void *> in_ptr(ni), out_ptr(no), out_host(no, nullptr), out_user(no, nullptr);
+    struct SmallInput {
+      size_t index, bytes, offset;
+      const void *host;
+    };
+    std::vector<SmallInput> small;   // pageable inputs that travel through the pinned block
+    size_t small_bytes = 0;
+    std::vector<char> dev_in(ni, 0);
+    bool any_host_in = false, any_dev_out = false;
     // host copies overlapped with the first / last step (synchronous API only)
     const Step *first = plan.steps.empty() ? nullptr : &plan.steps.front();
     const Step *last = plan.steps.empty() ? nullptr : &plan.steps.back();
@@ -475,13 +541,21 @@ struct dnnl_graph_compiler_executable {
       dnnl_graph_compiler_tensor *t = find(inputs, ni, i, lt.id);
       check_dims(t, lt);
       const size_t bytes = span_elems(lt) * dtype_bytes(lt.dtype);
-      if (on_device(t->data)) {
+      const Where w = where(t->data);
+      if (w == Where::DEVICE) {
         in_ptr[i] = t->data;
+        dev_in[i] = 1;
         if (long(i) == piped_in) piped_in = -1;
+      } else if (own_stream && w == Where::PAGEABLE && !lt.constant && small_bytes + padded(bytes) <= kSmallIn) {
+        if (long(i) == piped_in) piped_in = -1;
+        small.push_back(SmallInput{i, bytes, small_bytes, t->data});
+        small_bytes += padded(bytes);
+        any_host_in = true;
       } else if (long(i) == piped_in) {
         in_stage[i].reserve(bytes);
         in_ptr[i] = in_stage[i].ptr;
         piped_in_host = t->data;
+        any_host_in = true;
       } else {
         DeviceBuffer &b = in_stage[i];
         // GC_B200_CONST_CACHE=0: re-read constant tensors on every call, as the reference does (for callers that
@@ -500,16 +574,28 @@ struct dnnl_graph_compiler_executable {
             }
         }
         in_ptr[i] = b.ptr;
+        any_host_in = true;
       }
     }
+    if (small_bytes) {
+      small_in_host.reserve(small_bytes);
+      small_in.reserve(small_bytes);
+      for (const SmallInput &q : small) in_ptr[q.index] = static_cast<uint8_t *>(small_in.ptr) + q.offset;
+    }
+    size_t small_out = 0;
     for (size_t i = 0; i < no; ++i) {
       const LogicalTensor &lt = p.tensors.at(p.output_ids[i]);
       dnnl_graph_compiler_tensor *t = find(outputs, no, i, lt.id);
       check_dims(t, lt);
       const size_t bytes = size_t(lt.numel()) * dtype_bytes(lt.dtype);
-      if (on_device(t->data)) {
+      const Where w = where(t->data);
+      if (w == Where::DEVICE) {
         out_ptr[i] = t->data;
         if (long(i) == piped_out) piped_out = -1;
+        any_dev_out = true;
+      } else if (own_stream && long(i) != piped_out && small_out + padded(bytes) <= kSmallOut && host_writable[i]) {
+        out_user[i] = t->data;
+        small_out += padded(bytes);
       } else {
         out_stage[i].reserve(bytes);
         out_ptr[i] = out_stage[i].ptr;
@@ -520,10 +606,27 @@ struct dnnl_graph_compiler_executable {
     // being produced (or their memory still be in use) by work the caller queued on other streams;
     // order this call after all of it.
     if (own_stream) {
-      bool any_dev = false;
-      for (size_t i = 0; i < ni; ++i) any_dev |= (in_ptr[i] != in_stage[i].ptr);
-      for (size_t i = 0; i < no; ++i) any_dev |= (out_host[i] == nullptr);
+      bool any_dev = any_dev_out;
+      for (size_t i = 0; i < ni; ++i) any_dev |= dev_in[i] != 0;
       if (any_dev) GCB_CUDA(cudaDeviceSynchronize());
+    }
+    if (small_out) {
+      small_out_host.reserve(small_out);
+      size_t off = 0;
+      for (size_t i = 0; i < no; ++i)
+        if (out_user[i]) {
+          out_ptr[i] = small_out_host.ptr + off;
+          off += padded(size_t(p.tensors.at(p.output_ids[i]).numel()) * dtype_bytes(p.tensors.at(p.output_ids[i]).dtype));
+        }
+    }
+    // the block is filled tensor by tensor and sent on in pieces, so that the device reads one while the next is copied
+    for (size_t k = 0, sent = 0; k < small.size(); ++k) {
+      std::memcpy(small_in_host.ptr + small[k].offset, small[k].host, small[k].bytes);
+      const size_t end = small[k].offset + padded(small[k].bytes);
+      if (end > sent && (k + 1 == small.size() || end - sent >= (128 << 10))) {
+        fetch_pinned(static_cast<uint8_t *>(small_in.ptr) + sent, small_in_host.ptr + sent, end - sent, s);
+        sent = end;
+      }
     }
     auto addr = [&](size_t id) -> void * {
       const TensorSlot &sl = plan.slots.at(id);
@@ -544,9 +647,8 @@ struct dnnl_graph_compiler_executable {
     }
     if (piped_out >= 0 && !tc_ok(*last)) piped_out = -1;
     // ---- every tensor in device memory: the launch list does not depend on anything but the addresses
-    bool all_dev = true;
-    for (size_t i = 0; i < ni; ++i) all_dev &= (in_ptr[i] != in_stage[i].ptr || in_stage[i].ptr == nullptr);
-    for (size_t i = 0; i < no; ++i) all_dev &= (out_host[i] == nullptr);
+    bool all_dev = !any_host_in;
+    for (size_t i = 0; i < no; ++i) all_dev &= (out_host[i] == nullptr && out_user[i] == nullptr);
     static const bool graphs_on = [] { const char *e = std::getenv("GC_B200_GRAPHS"); return !(e && e[0] == '0'); }();
     bool replayed = false;
     if (all_dev && graphs_on && plan.steps.size() > 1) {
@@ -649,18 +751,16 @@ struct dnnl_graph_compiler_executable {
         GCB_CUDA(cudaMemcpyAsync(out_host[i], out_ptr[i], size_t(lt.numel()) * dtype_bytes(lt.dtype), cudaMemcpyDeviceToHost, s));
       }
     bool any_host = false;
-    for (void *h : out_host) any_host |= (h != nullptr);
+    for (size_t i = 0; i < no; ++i) any_host |= out_host[i] != nullptr || out_user[i] != nullptr;
     if (sync || any_host) {
-      // the error word travels behind the results on the same stream: one wait covers both
-      GCB_CUDA(cudaMemcpyAsync(host_code, device_state().d_error, sizeof(int), cudaMemcpyDeviceToHost, s));
       GCB_CUDA(cudaStreamSynchronize(s));
       if (piped_out >= 0) GCB_CUDA(cudaStreamSynchronize(copy_out));
-      const int code = *host_code;
-      if (code) {
-        GCB_CUDA(cudaMemset(device_state().d_error, 0, sizeof(int)));
+      if (const int code = device_state().take_error()) {
         gcLogE("device error word = ", code, " after execute");
         throw std::runtime_error("a kernel gave up a bounded wait (code " + std::to_string(code) + ")");
       }
+      for (size_t i = 0; i < no; ++i)
+        if (out_user[i]) std::memcpy(out_user[i], out_ptr[i], size_t(p.tensors.at(p.output_ids[i]).numel()) * dtype_bytes(p.tensors.at(p.output_ids[i]).dtype));
       if (plan.guard_bytes) {
         std::string what;
         const int bad = check_guards(&what);
@@ -671,6 +771,11 @@ struct dnnl_graph_compiler_executable {
         }
       }
     }
+  }
+
+  bool in_small_out(const void *q) const {
+    const uint8_t *b = static_cast<const uint8_t *>(q);
+    return small_out_host.ptr && b >= small_out_host.ptr && b < small_out_host.ptr + small_out_host.bytes;
   }
 
   template <class Addr>
@@ -688,6 +793,7 @@ struct dnnl_graph_compiler_executable {
         m.out_kind = OUT_BF16; m.out = addr(st.out[0]);
         m.bias_kind = bias ? BIAS_BF16 : BIAS_NONE; m.bias = bias; m.relu = st.relu;
         m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;
+        m.plain_stores = in_small_out(m.out);
         const size_t need = matmul_pack_bytes(m);
         if (need && need <= pack.bytes) matmul_bf16_packed(m, pack.ptr, s);
         else matmul_bf16_any_layout(m, s);
@@ -733,6 +839,7 @@ struct dnnl_graph_compiler_executable {
       m.bias = st.has_bias ? addr(st.in[3]) : nullptr;
       m.acc_dump = st.out.size() > 1 ? static_cast<int32_t *>(addr(st.out[1])) : nullptr;
       m.relu = st.relu;
+      m.plain_stores = in_small_out(m.out);
       if (!(tma_compatible(m.A, st.K, 1) && tma_compatible(m.B, st.N, 1)))
         throw std::logic_error("QuantizedMatMul needs K and N to be multiples of 16");
       m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;

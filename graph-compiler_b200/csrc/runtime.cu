@@ -36,9 +36,10 @@ DeviceState &device_state() {
       throw CudaError("this library is built for sm_100a only; device is sm_" + std::to_string(prop.major) +
                       std::to_string(prop.minor));
     d.sm_count = prop.multiProcessorCount;
-    GCB_CUDA(cudaMalloc(&d.d_error, 64));
-    GCB_CUDA(cudaMemset(d.d_error, 0, 64));
-    d.d_zero = d.d_error + 8;
+    GCB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&d.d_error), 64, cudaHostAllocMapped | cudaHostAllocPortable));
+    std::memset(d.d_error, 0, 64);
+    GCB_CUDA(cudaMalloc(&d.d_zero, 64));
+    GCB_CUDA(cudaMemset(d.d_zero, 0, 64));
     d.device = dev;
   }
   return d;
@@ -62,11 +63,8 @@ void *DeviceState::ensure_workspace(size_t bytes) {
 
 int read_device_error(cudaStream_t stream) {
   DeviceState &d = device_state();
-  int h = 0;
-  GCB_CUDA(cudaMemcpyAsync(&h, d.d_error, sizeof(int), cudaMemcpyDeviceToHost, stream));
   GCB_CUDA(cudaStreamSynchronize(stream));
-  if (h != 0) GCB_CUDA(cudaMemsetAsync(d.d_error, 0, sizeof(int), stream));
-  return h;
+  return d.take_error();
 }
 
 // ----------------------------------------------------------------------------- tensor maps
@@ -468,7 +466,7 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
     const bool plain = p.out_kind == OUT_BF16          ? (p.bias_kind == BIAS_NONE || p.bias_kind == BIAS_BF16)
                        : p.out_kind == OUT_DEQUANT_F32 ? (p.bias_kind == BIAS_NONE || p.bias_kind == BIAS_F32)
                                                        : ((p.out_kind == OUT_F32 || p.out_kind == OUT_S32) && p.bias_kind == BIAS_NONE && !p.relu);
-    if (plain && tma_compatible(p.out, p.ld_out, esz) && (!split || (size_t(p.split_stride) * esz) % 16 == 0)) {
+    if (plain && (split || !a.plain_stores) && tma_compatible(p.out, p.ld_out, esz) && (!split || (size_t(p.split_stride) * esz) % 16 == 0)) {
       const ElemType ct = p.out_kind == OUT_BF16 ? ElemType::BF16 : (p.out_kind == OUT_S32 ? ElemType::S32 : ElemType::F32);
       p.tmC = make_tmap_3d(ct, p.out, uint64_t(a.N), uint64_t(a.M), uint64_t(std::max(1, p.splits)), uint64_t(p.ld_out) * esz,
                            split ? uint64_t(p.split_stride) * esz : uint64_t(a.M) * uint64_t(p.ld_out) * esz, 128 / esz, 32, 1);

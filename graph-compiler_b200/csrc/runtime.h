@@ -29,7 +29,16 @@ struct CudaError : std::runtime_error {
 struct DeviceState {
   int device = -1;
   int sm_count = 0;
-  int *d_error = nullptr;          // device word written by kernels on a bounded-wait time-out
+  // Word written by kernels on a bounded-wait time-out.  Pinned host memory that the device addresses directly: kernels
+  // touch it only when they give up, and after a stream synchronisation the host reads it without a copy (a copy behind
+  // every synchronous call cost 4 us).
+  int *d_error = nullptr;
+  int take_error() {               // reads and clears; the kernels in question must have completed
+    volatile int *w = d_error;
+    const int code = *w;
+    if (code) *w = 0;
+    return code;
+  }
   int *d_zero = nullptr;           // device word that stays zero (the wait self-test waits on it)
   // Split-K partial planes of the direct launchers (executables bring their own scratch).  ONE block per
   // device, shared by every stream and thread: launches that may split K and overlap on the GPU must be
@@ -108,6 +117,7 @@ struct MatmulArgs {
                                 // (plane = peer_plane * peer_splits + split; the owner's buffer holds n_peers * peer_splits planes)
   void *const *peer_out = nullptr;
   int peer_multicast = 0;       // 1: n_peers == 1 and peer_out[0] is an NVLink multicast address of all ranks' buffers
+  int plain_stores = 0;         // 1: `out` is written with ordinary stores (memory of the host)
   const MatmulConfig *force = nullptr; // optional override
   void *scratch = nullptr;      // optional caller-provided split-K scratch (else the device workspace)
   size_t scratch_bytes = 0;

@@ -203,7 +203,6 @@ struct gcb200_tp_mlp {
   void *splitk = nullptr;
   size_t splitk_bytes = 0;
   cudaStream_t stream = nullptr; // host-buffer path
-  int *host_code = nullptr;
   // optional timeline of one eagerly launched step: an event after every launch (see gcb200_tp_mlp_timeline)
   std::vector<cudaEvent_t> marks;
   std::vector<std::string> mark_names;
@@ -249,7 +248,6 @@ struct gcb200_tp_mlp {
     if (splitk) cudaFree(splitk);
     if (trace) cudaFree(trace);
     if (stream) cudaStreamDestroy(stream);
-    if (host_code) cudaFreeHost(host_code);
   }
 
   void plan_row_layers(int sm_count) {
@@ -305,8 +303,6 @@ struct gcb200_tp_mlp {
       GCB_CUDA(cudaMemset(trace, 0, words * sizeof(unsigned long long)));
     }
     GCB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    GCB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&host_code), sizeof(int), cudaHostAllocDefault));
-    *host_code = 0;
     ready = true;
   }
 
@@ -576,15 +572,9 @@ GCB_EXPORT int gcb200_tp_mlp_execute(gcb200_tp_mlp *t, const void *x_host, void 
       t->enqueue_scatter(q);
       t->enqueue_step(t->x_in[size_t(t->rank)], true, q);
       if (y_host) GCB_CUDA(cudaMemcpyAsync(y_host, t->result(), out_bytes, cudaMemcpyDeviceToHost, q));
-      GCB_CUDA(cudaMemcpyAsync(t->host_code, d.d_error, sizeof(int), cudaMemcpyDeviceToHost, q));
     });
     GCB_CUDA(cudaStreamSynchronize(s));
-    const int code = *t->host_code;
-    if (code) {
-      GCB_CUDA(cudaMemset(d.d_error, 0, sizeof(int)));
-      *t->host_code = 0;
-      throw CudaError("a kernel gave up a bounded wait (code " + std::to_string(code) + ")");
-    }
+    if (const int code = d.take_error()) throw CudaError("a kernel gave up a bounded wait (code " + std::to_string(code) + ")");
     return GCB200_OK;
   } catch (...) {
     return guard_status(std::current_exception());
