@@ -16,14 +16,14 @@
 #include <string>
 #include <vector>
 
-#include <cuda_fp16.h>
-
 #include "../../include/dnnl_graph_compiler.h"
 #include "../../include/gc_b200.h"
 #include "attention.h"
+#include "elementwise.cuh"
 #include "graph.h"
 #include "log.h"
 #include "memplan.h"
+#include "rowprog.h"
 #include "runtime.h"
 #include "sm100_ptx.cuh"
 
@@ -70,31 +70,11 @@ __device__ __forceinline__ long long ew_offset(const EwParams &p, long long i, i
   }
 }
 
-__device__ __forceinline__ float ew_load(const void *p, long long i, int dt) {
-  if (dt == 0) return reinterpret_cast<const float *>(p)[i];
-  if (dt == 1) return bf16_bits_to_f32(reinterpret_cast<const uint16_t *>(p)[i]);
-  return __half2float(reinterpret_cast<const __half *>(p)[i]);
-}
-// Every bf16/f16 op rounds once on store: the reference evaluates low-precision
-// elementwise ops as extf -> f32 op -> truncf (lib/gc/Transforms/Pipeline.cpp:81-90).
-__device__ __forceinline__ void ew_store(void *p, long long i, int dt, float v) {
-  if (dt == 0) reinterpret_cast<float *>(p)[i] = v;
-  else if (dt == 1) reinterpret_cast<uint16_t *>(p)[i] = uint16_t(f32_to_bf16_bits(v));
-  else reinterpret_cast<__half *>(p)[i] = __float2half_rn(v);
-}
-
 __global__ void binary_kernel(EwParams p, const void *a, const void *b, void *o) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
     const long long oa = ew_offset(p, i, p.mode_a, p.sa), ob = ew_offset(p, i, p.mode_b, p.sb);
     const float x = ew_load(a, oa, p.dt_a), y = ew_load(b, ob, p.dt_b);
-    float v;
-    switch (p.fn) {
-    case 0: v = __fadd_rn(x, y); break;
-    case 1: v = __fsub_rn(x, y); break;
-    case 2: v = __fmul_rn(x, y); break;
-    default: v = __fdiv_rn(x, y); break;
-    }
-    ew_store(o, i, p.dt_o, v);
+    ew_store(o, i, p.dt_o, ew_binary(p.fn, x, y));
   }
 }
 
@@ -102,22 +82,7 @@ __global__ void unary_kernel(EwParams p, const void *a, void *o) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < p.total; i += (long long)gridDim.x * blockDim.x) {
     const long long oa = ew_offset(p, i, p.mode_a, p.sa);
     const float x = ew_load(a, oa, p.dt_a);
-    float v;
-    switch (p.fn) {
-    case 0: v = (x != x) ? x : (x > 0.f ? x : 0.f); break;       // max(x, 0), NaN propagates
-    case 1: v = __fdiv_rn(1.f, __fadd_rn(1.f, expf(-x))); break; // 1 / (1 + exp(-x))
-    case 2:
-      if (p.beta == 2.f) v = __fmul_rn(x, x);
-      else if (p.beta == 1.f) v = x;
-      else if (p.beta == 0.5f) v = sqrtf(x);
-      else if (p.beta == 3.f) v = __fmul_rn(__fmul_rn(x, x), x);
-      else v = powf(x, p.beta);
-      break;
-    case 4: v = expf(x); break;
-    case 5: v = -x; break;
-    default: v = x; break;
-    }
-    ew_store(o, i, p.dt_o, v);
+    ew_store(o, i, p.dt_o, ew_unary(p.fn, p.beta, x));
   }
 }
 
@@ -206,9 +171,9 @@ __global__ void __launch_bounds__(256) reduce_block_kernel(ReduceParams p, const
 // thread, up to 64 blocks of 256) for the bus rate at its latency; a copy engine has the same rate but starts later and
 // hands over to the next kernel through a semaphore.  Both ends are multiples of 16 bytes.
 __global__ void __launch_bounds__(256) fetch_pinned_kernel(uint4 *dst, const uint4 *src, int n) {
+  pdl_wait();
   pdl_launch_dependents();
   for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) dst[i] = __ldcs(src + i);
-  pdl_wait();   // what runs behind this kernel runs behind everything ahead of it
 }
 static void fetch_pinned(void *dst, const void *src, size_t bytes, cudaStream_t s) {
   const int n = int(bytes / 16);
@@ -323,11 +288,24 @@ struct dnnl_graph_compiler_executable {
   static constexpr int kCanary = 0xA5;
   mutable DeviceBuffer splitk;          // split-K partial planes of this executable's matmul steps (they run one after
                                         // another on one stream, so one block sized for the largest request serves all)
+  mutable size_t shared_planes = 0;     // where the part shared by all steps begins, behind the planes that stay
   mutable DeviceBuffer pack;            // likewise: packed copies of operands whose rows are no whole number of 16 bytes
 
   std::vector<char> host_writable;      // per output: its step may write it in host memory (nothing reads it back, and
                                         // the step is a kernel with plain stores)
+  std::vector<RowGroup> groups;         // runs of elementwise steps that execute as one kernel
+  std::vector<int> group_at;            // per step: the run that starts there, or -1
+  std::vector<char> defers;             // per step: a matmul whose K-split planes a run sums
+  mutable std::vector<size_t> plane_at, plane_room;   // per such step: its planes' place in the split-K block
   explicit dnnl_graph_compiler_executable(const std::string &json) : plan(build_plan(read_partition(json))) {
+    static const bool fuse = [] { const char *e = std::getenv("GC_B200_FUSE"); return !(e && e[0] == '0'); }();
+    if (fuse) groups = plan_row_groups(plan);
+    group_at.assign(plan.steps.size(), -1);
+    defers.assign(plan.steps.size(), 0);
+    for (size_t i = 0; i < groups.size(); ++i) {
+      group_at[size_t(groups[i].first)] = int(i);
+      for (int m : groups[i].deferred) defers[size_t(m)] = 1;
+    }
     for (size_t id : plan.part.output_ids) {
       bool ok = true;
       for (const Step &st : plan.steps) {
@@ -372,16 +350,26 @@ struct dnnl_graph_compiler_executable {
       // split-K scratch of every matmul step, as the selector sees the shapes on this device (whole step and,
       // where the step may run as row blocks, one block); a configuration recorded later that needs more
       // falls back to the per-device workspace inside matmul_tc
-      size_t need = 0;
-      for (const Step &st : plan.steps) {
+      size_t need = 0, kept = 0;   // kept: planes that outlive their matmul step, each with a place of its own
+      plane_at.assign(plan.steps.size(), 0);
+      plane_room.assign(plan.steps.size(), 0);
+      for (size_t i = 0; i < plan.steps.size(); ++i) {
+        const Step &st = plan.steps[i];
         if (st.kind != StepKind::MATMUL && st.kind != StepKind::QMATMUL) continue;
+        if (defers[i]) {
+          plane_at[i] = kept;
+          plane_room[i] = padded(matmul_scratch_bytes(st.M, st.N, st.K, 2, 2, d.sm_count));
+          kept += plane_room[i];
+          continue;
+        }
         const bool q = st.kind == StepKind::QMATMUL;
         if (!q && plan.part.tensors.at(st.in[0]).dtype != DType::BF16) continue;
         need = std::max(need, matmul_scratch_bytes(st.M, st.N, st.K, q ? 1 : 2, q ? 4 : 2, d.sm_count));
         if (!q && rows_chunkable(st))
           need = std::max(need, matmul_scratch_bytes(st.M / kRowChunks, st.N, st.K, 2, 2, d.sm_count));
       }
-      if (need) splitk.reserve(need);
+      shared_planes = kept;
+      if (need + kept) splitk.reserve(need + kept);
       size_t packed = 0;
       for (const Step &st : plan.steps) {
         if (st.kind != StepKind::MATMUL || plan.part.tensors.at(st.in[0]).dtype != DType::BF16) continue;
@@ -445,7 +433,7 @@ struct dnnl_graph_compiler_executable {
     m.B = b; m.M = rows; m.N = st.N; m.K = st.K; m.trans_a = 0; m.trans_b = st.trans_b;
     m.out_kind = OUT_BF16; m.out = static_cast<uint8_t *>(out) + size_t(r0) * size_t(st.N) * 2;
     m.bias_kind = bias ? BIAS_BF16 : BIAS_NONE; m.bias = bias; m.relu = st.relu;
-    m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;
+    m.scratch = static_cast<uint8_t *>(splitk.ptr) + shared_planes; m.scratch_bytes = splitk.bytes - shared_planes;
     matmul_tc(m, s);
   }
 
@@ -685,7 +673,7 @@ struct dnnl_graph_compiler_executable {
             bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
             if (ok) {
               try {
-                for (const Step &st : plan.steps) run_step(st, addr, in_ptr, s);
+                run_steps(0, plan.steps.size(), addr, in_ptr, s);
               } catch (...) {
                 ok = false;
               }
@@ -717,7 +705,9 @@ struct dnnl_graph_compiler_executable {
       const Step &st = plan.steps[k];
       const bool chunk_in = (k == 0 && piped_in >= 0), chunk_out = (k + 1 == plan.steps.size() && piped_out >= 0);
       if (!chunk_in && !chunk_out) {
-        run_step(st, addr, in_ptr, s);
+        const size_t end = piped_out >= 0 ? plan.steps.size() - 1 : plan.steps.size();
+        run_steps(k, end, addr, in_ptr, s);
+        k = end - 1;
         continue;
       }
       // the step runs as kRowChunks row blocks: block c starts when its rows of A have arrived, and its
@@ -778,8 +768,55 @@ struct dnnl_graph_compiler_executable {
     return small_out_host.ptr && b >= small_out_host.ptr && b < small_out_host.ptr + small_out_host.bytes;
   }
 
+  // Steps [begin, end) in order, elementwise runs as one kernel where their tensors are 16-byte aligned.
   template <class Addr>
-  void run_step(const Step &st, Addr &addr, const std::vector<void *> &in_ptr, cudaStream_t s) const {
+  void run_steps(size_t begin, size_t end, Addr &addr, const std::vector<void *> &in_ptr, cudaStream_t s) const {
+    // Whether this call has launched something: every kernel of this library lets the next one start only behind its own
+    // wait for the kernel ahead, so from the second launch on all work that was queued before the call (and the
+    // copies of its arguments) is done when a kernel starts, and arguments may be fetched at once.
+    bool behind_own = begin > 0;
+    std::vector<int> planes(plan.steps.size(), 0);   // deferred matmuls: partial planes left behind (0: finished result)
+    for (size_t k = begin; k < end; ++k) {
+      if (group_at[k] >= 0) {
+        const RowGroup &g = groups[size_t(group_at[k])];
+        RowProgram p = g.prog;
+        bool ok = size_t(g.last) < end;
+        for (size_t i = 0; i < g.ids.size(); ++i) {
+          p.ptr[i] = addr(g.ids[i]);
+          p.planes[i] = 0;
+          ok &= (reinterpret_cast<uintptr_t>(p.ptr[i]) & 15) == 0;
+        }
+        for (int m : g.deferred) {
+          const Step &ms = plan.steps[size_t(m)];
+          if (planes[size_t(m)] == 0) continue;
+          const size_t i = size_t(std::find(g.ids.begin(), g.ids.end(), ms.out[0]) - g.ids.begin());
+          p.ptr[i] = static_cast<uint8_t *>(splitk.ptr) + plane_at[size_t(m)];
+          p.planes[i] = planes[size_t(m)];
+          p.plane_stride[i] = (long long)ms.M * ms.N;
+        }
+        if (ok) {
+          launch_row_program(p, s);
+          behind_own = true;
+          k = size_t(g.last);
+          continue;
+        }
+        for (int m : g.deferred)   // one by one after all: finish the sums first
+          if (planes[size_t(m)]) {
+            const Step &ms = plan.steps[size_t(m)];
+            reduce_planes(static_cast<uint8_t *>(splitk.ptr) + plane_at[size_t(m)], planes[size_t(m)], ms.M * ms.N, addr(ms.out[0]), ms.M, ms.N,
+                          OUT_BF16, BIAS_NONE, nullptr, nullptr, nullptr, nullptr, 0, s);
+          }
+      }
+      run_step(plan.steps[k], addr, in_ptr, s, defers[k] ? &planes[k] : nullptr, plane_at[k], plane_room[k], behind_own);
+      const StepKind kind = plan.steps[k].kind;
+      behind_own |= kind == StepKind::MATMUL || kind == StepKind::QMATMUL || kind == StepKind::SDPA;
+    }
+  }
+
+  // planes: the step may leave its K-split partial planes in [at, at + room) of the split-K block and report their number.
+  template <class Addr>
+  void run_step(const Step &st, Addr &addr, const std::vector<void *> &in_ptr, cudaStream_t s, int *planes = nullptr, size_t at = 0,
+                size_t room = 0, bool behind_own = false) const {
     const Partition &p = plan.part;
     switch (st.kind) {
     case StepKind::MATMUL: {
@@ -792,7 +829,10 @@ struct dnnl_graph_compiler_executable {
         m.A = a; m.B = b; m.M = st.M; m.N = st.N; m.K = st.K; m.trans_a = st.trans_a; m.trans_b = st.trans_b;
         m.out_kind = OUT_BF16; m.out = addr(st.out[0]);
         m.bias_kind = bias ? BIAS_BF16 : BIAS_NONE; m.bias = bias; m.relu = st.relu;
-        m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;
+        m.scratch = static_cast<uint8_t *>(splitk.ptr) + (planes ? at : shared_planes);
+        m.scratch_bytes = planes ? room : splitk.bytes - shared_planes;
+        m.early_weights = behind_own && plan.slots.at(st.in[1]).where == TensorSlot::INPUT;
+        m.keep_planes = planes;
         m.plain_stores = in_small_out(m.out);
         const size_t need = matmul_pack_bytes(m);
         if (need && need <= pack.bytes) matmul_bf16_packed(m, pack.ptr, s);
@@ -822,7 +862,7 @@ struct dnnl_graph_compiler_executable {
         m.out_kind = OUT_S32; m.out = addr(st.out[0]);
         if (!(tma_compatible(m.A, st.K, 1) && tma_compatible(m.B, st.N, 1)))
           throw std::logic_error("QuantizedMatMul needs K and N to be multiples of 16");
-        m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;
+        m.scratch = static_cast<uint8_t *>(splitk.ptr) + shared_planes; m.scratch_bytes = splitk.bytes - shared_planes;
         matmul_tc(m, s);
         if (st.zp_a != 0) {
           const long long total = (long long)st.M * st.N;
@@ -842,7 +882,7 @@ struct dnnl_graph_compiler_executable {
       m.plain_stores = in_small_out(m.out);
       if (!(tma_compatible(m.A, st.K, 1) && tma_compatible(m.B, st.N, 1)))
         throw std::logic_error("QuantizedMatMul needs K and N to be multiples of 16");
-      m.scratch = splitk.ptr; m.scratch_bytes = splitk.bytes;
+      m.scratch = static_cast<uint8_t *>(splitk.ptr) + shared_planes; m.scratch_bytes = splitk.bytes - shared_planes;
       matmul_tc(m, s);
       break;
     }

@@ -102,8 +102,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // Everything above touched only shared and tensor memory and may overlap the tail of the kernel
   // ahead in the stream; from here on operands are read and results written.
   if (blockIdx.x == 0 && threadIdx.x == 0) trace_store(p.trace, 0);
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) trace_store(p.trace, 1);
 
   if (warp == 0 || warp == 6) {

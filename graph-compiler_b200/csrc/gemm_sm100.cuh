@@ -16,6 +16,7 @@ enum ErrCode : int {
   ERR_WAIT_TMEM_FULL = 4,  // epilogue: an accumulator was never committed
   ERR_WAIT_DRAIN = 5,      // tear-down: an issued copy did not land
   ERR_WAIT_PEER = 6,       // a cross-GPU counter (rows landed / partial sums landed) never reached its target
+  ERR_WAIT_PARTS = 8,      // few-rows form: a CTA of the cluster never handed over its partial sums
   ERR_SELFTEST = 7,        // the wait self-test: a wait nobody satisfies ran out, as intended
 };
 

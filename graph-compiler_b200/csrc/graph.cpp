@@ -451,6 +451,23 @@ Plan build_plan(Partition part) {
     plan.steps.push_back(std::move(st));
   }
 
+  // ---- elementwise steps run together where they can (rowprog.h): a matmul that does not need the elementwise steps
+  // ahead of it moves in front of them, so that runs interrupted by one become whole
+  auto elementwise = [](const Step &st) {
+    return st.kind == StepKind::BINARY || st.kind == StepKind::UNARY || st.kind == StepKind::REDUCE;
+  };
+  for (size_t i = 1; i < plan.steps.size(); ++i) {
+    if (plan.steps[i].kind != StepKind::MATMUL && plan.steps[i].kind != StepKind::QMATMUL) continue;
+    size_t j = i;
+    auto independent = [&](const Step &before) {
+      for (size_t id : before.out)
+        if (std::find(plan.steps[i].in.begin(), plan.steps[i].in.end(), id) != plan.steps[i].in.end()) return false;
+      return elementwise(before);
+    };
+    while (j > 0 && independent(plan.steps[j - 1])) --j;
+    if (j < i && j > 0) std::rotate(plan.steps.begin() + long(j), plan.steps.begin() + long(i), plan.steps.begin() + long(i) + 1);
+  }
+
   // ---- storage: arguments and results are the caller's; everything else lives in the arena
   size_t guard = 0;
   if (const char *g = std::getenv("GC_B200_GUARD")) {
@@ -497,6 +514,22 @@ Plan build_plan(Partition part) {
       // arena belongs to the executable, from one call to the next).
       lives.push_back(BufferLife{size_t(st.N) * 4 + 2 * guard, 0, int(plan.steps.size()) - 1});
     }
+  }
+  // a run of elementwise steps may execute as one: what it reads stays alive to its end, what leaves it is born at its
+  // start
+  for (size_t b = 0; b < plan.steps.size();) {
+    size_t e = b;
+    while (e < plan.steps.size() && elementwise(plan.steps[e])) ++e;
+    if (e == b) {
+      ++b;
+      continue;
+    }
+    for (BufferLife &l : lives) {
+      const int first = int(b), last = int(e) - 1;
+      if (l.first < first && l.last >= first && l.last < last) l.last = last;
+      if (l.first > first && l.first <= last && l.last > last) l.first = first;
+    }
+    b = e;
   }
   // an output may also be consumed by a later op.  Results are written densely: an output declared with
   // other strides, or an output that is one of the partition's own arguments (nothing here produces it),

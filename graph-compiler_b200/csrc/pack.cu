@@ -18,8 +18,8 @@ namespace {
 // are loaded and shifted by half a word where needed; words that lie partly outside the matrix are put together from
 // single elements.
 __global__ void __launch_bounds__(256) pack_rows_kernel(const uint16_t *src, uint4 *dst, long long rows, int cols, int chunks) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   const long long total = rows * chunks;
   const uintptr_t first = reinterpret_cast<uintptr_t>(src), last = reinterpret_cast<uintptr_t>(src + rows * cols);
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {

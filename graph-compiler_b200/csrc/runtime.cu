@@ -2,6 +2,7 @@
 // planning and the small helper kernels (split-K reduction + epilogue, int8
 // column sums, exact-order SIMT matmul).
 #include "runtime.h"
+#include "gemm_decode.h"
 #include "tune_cache.h"
 
 #include <algorithm>
@@ -261,7 +262,71 @@ MatmulConfig model_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_byte
 
 size_t matmul_scratch_bytes(int64_t M, int64_t N, int64_t K, int dtype_bytes, int out_bytes, int sm_count) {
   const MatmulConfig c = select_matmul_config(M, N, K, dtype_bytes, out_bytes, sm_count);
+  if (c.swapped) return 0;
   return c.splits > 1 ? size_t(c.splits) * size_t(M) * size_t(N) * 4 : 0;
+}
+
+// CTAs that share a tile's K range.  A K block of a tile (16 KB of weights) takes a CTA 0.26 us when it is not held up by
+// the others, 6.2 TB/s bound them all, and a split costs about 1 us (partial sums exchanged in the cluster): the split with
+// the cheapest sum over the rounds, each CTA with four K blocks at least.  All measured at 32 x 11008 x 4096 and around it.
+static int decode_split(int tiles, int k_blocks, bool int8, int device, int *at_once) {
+  int best = 1;
+  double best_t = 1e30;
+  for (int split = 1; split <= 8; ++split) {
+    if (split > 1 && k_blocks < 4 * split) break;
+    const int per = ceil_div(k_blocks, split);
+    if (split > 1 && per * (split - 1) >= k_blocks) continue;   // the last CTA would have nothing to do
+    const int clusters = decode_clusters_at_once(int8, device, split);
+    if (clusters < 1) continue;
+    const int rounds = ceil_div(tiles, clusters), active = std::min(tiles, clusters) * split;
+    const double t = rounds * per * std::max(0.26, active * 16384 / 6.2e6) + (split > 1 ? 1.0 + 0.1 * split : 0.0);
+    if (t < best_t) {
+      best_t = t;
+      best = split;
+      *at_once = clusters;
+    }
+  }
+  return best;
+}
+
+static void matmul_decode(const MatmulArgs &a, cudaStream_t stream) {
+  DeviceState &dev = device_state();
+  const int eb = a.int8 ? 1 : 2;
+  DecodeParams p{};
+  const bool w_mn = a.trans_b == 0, x_mn = a.trans_a != 0;
+  p.bk_elems = 128 / eb;
+  p.k_blocks = ceil_div(a.K, p.bk_elems);
+  p.tiles = ceil_div(a.N, 128);
+  int clusters = 1;
+  p.split = decode_split(p.tiles, p.k_blocks, a.int8 != 0, dev.device, &clusters);
+  p.parts_bytes = p.split > 1 ? uint32_t(a.M) * 512u : 0u;
+  p.BN = std::max(16, ceil_div(a.M, 16) * 16);
+  p.early_weights = a.early_weights;
+  p.w = operand_geom(w_mn, 128, eb, 1);
+  p.x = operand_geom(x_mn, p.BN, eb, 1);
+  const CUtensorMap tmW = operand_tmap(p.w, a.int8 ? ElemType::S8 : ElemType::BF16, eb, a.B, a.N, a.K, 128, 1, a.ldb);
+  const CUtensorMap tmX = operand_tmap(p.x, a.int8 ? ElemType::U8 : ElemType::BF16, eb, a.A, a.M, a.K, p.BN, 1, a.lda);
+  p.idesc = umma_instr_desc(a.int8 ? 2u : 1u, 1u, a.int8 ? 0u : 1u, w_mn ? 1u : 0u, x_mn ? 1u : 0u, 128u, uint32_t(p.BN));
+  p.tmem_cols = 32;
+  while (p.tmem_cols < uint32_t(2 * p.BN)) p.tmem_cols <<= 1;
+  p.stages = decode_stages(p);
+  p.out_kind = a.out_kind;
+  p.out = a.out;
+  p.ld_out = a.ld_out ? a.ld_out : a.N;
+  p.bias_kind = a.bias_kind;
+  p.bias = a.bias;
+  p.scale = a.scale;
+  p.comp = a.comp;
+  p.acc_dump = a.acc_dump;
+  p.ld_dump = a.N;
+  p.relu = a.relu;
+  p.out_rows = int(a.M);
+  p.out_cols = int(a.N);
+  p.error = dev.d_error;
+  const int grid = std::min(p.tiles, clusters) * p.split;
+  cudaError_t e = a.int8 ? launch_gemm_decode<1>(tmW, tmX, p, grid, dev.device, stream) : launch_gemm_decode<0>(tmW, tmX, p, grid, dev.device, stream);
+  if (e != cudaSuccess) throw CudaError(std::string("few-rows gemm launch: ") + cudaGetErrorString(e));
+  count_launch();
 }
 
 // ----------------------------------------------------------------------------- matmul planning
@@ -335,6 +400,10 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   const int max_splits = (a.n_peers > 0) ? 1 : 8;
   MatmulConfig cfg = a.force ? *a.force : select_matmul_config(a.M, a.N, a.K, eb, out_bytes, dev.sm_count, max_splits);
   const int64_t ld_out = a.ld_out ? a.ld_out : a.N;
+  if (cfg.swapped && !a.force && a.n_peers == 0 && !a.wait_counter && !a.trace) {
+    matmul_decode(a, stream);
+    return;
+  }
 
   GemmParams p{};
   p.K = int(a.K);
@@ -539,7 +608,9 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   }
   if (e != cudaSuccess) throw CudaError(std::string("gemm launch: ") + cudaGetErrorString(e));
   count_launch();
-  if (split) {
+  if (split && a.keep_planes && planes == a.scratch) {
+    *a.keep_planes = cfg.splits;
+  } else if (split) {
     if (ld_out != a.N) throw std::invalid_argument("split-K with a strided output is not supported");
     reduce_planes(planes, cfg.splits, a.M * a.N, a.out, a.M, a.N, a.out_kind, a.bias_kind, a.bias, a.scale, a.comp,
                   a.acc_dump, a.relu, stream);
@@ -595,8 +666,8 @@ __global__ void reduce_planes_kernel(const void *parts, int nparts, long long pl
 __global__ void __launch_bounds__(256)
 reduce_planes_bf16x4_kernel(const float4 *parts, int nparts, long long plane4, uint2 *out, long long total4, int n4,
                             const uint2 *bias, int relu) {
-  pdl_launch_dependents();
   pdl_wait();   // the planes come from the kernel ahead in the stream
+  pdl_launch_dependents();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total4; i += (long long)gridDim.x * blockDim.x) {
     // four planes' loads in flight before the first add (additions stay in split order)
     float4 s = parts[i];
@@ -629,8 +700,8 @@ struct PeerPtrs { uint2 *p[8]; };
 __global__ void __launch_bounds__(256)
 reduce_slice_bcast_kernel(const float4 *parts, int nparts, long long plane4, long long total4, int n4, const uint2 *bias,
                           int relu, PeerPtrs out, int n_peers, long long dst4) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total4; i += (long long)gridDim.x * blockDim.x) {
     float4 s = parts[i];
     for (int k = 1; k < nparts; ++k) {

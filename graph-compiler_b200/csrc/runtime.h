@@ -78,7 +78,7 @@ struct MatmulConfig {
 MatmulConfig select_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_bytes, int out_bytes, int sm_count, int max_splits = 8);
 // The fitted time model alone (select_matmul_config consults the measured configurations of tune_cache.h first).
 MatmulConfig model_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_bytes, int out_bytes, int sm_count, int max_splits = 8);
-// Bytes of f32 / s32 split-K partial planes the selected configuration of this shape needs (0: no split).
+// Bytes of f32 / s32 partial sums the selected configuration of this shape needs (0: no split).
 size_t matmul_scratch_bytes(int64_t M, int64_t N, int64_t K, int dtype_bytes, int out_bytes, int sm_count);
 // Whether the TMA path can take this operand layout (16-byte aligned base and row pitch).
 bool tma_compatible(const void *ptr, int64_t row_elems, int elem_bytes);
@@ -117,10 +117,13 @@ struct MatmulArgs {
                                 // (plane = peer_plane * peer_splits + split; the owner's buffer holds n_peers * peer_splits planes)
   void *const *peer_out = nullptr;
   int peer_multicast = 0;       // 1: n_peers == 1 and peer_out[0] is an NVLink multicast address of all ranks' buffers
+  int early_weights = 0;        // few-rows form: no work in flight on the device writes B (see gemm_decode_sm100.cu)
   int plain_stores = 0;         // 1: `out` is written with ordinary stores (memory of the host)
   const MatmulConfig *force = nullptr; // optional override
   void *scratch = nullptr;      // optional caller-provided split-K scratch (else the device workspace)
   size_t scratch_bytes = 0;
+  int *keep_planes = nullptr;   // K split with room in `scratch`: leave the partial planes there and report their number
+                                // instead of reducing them
   // cross-GPU hand-off (see GemmParams): counters to add to after the row scatter, counter to wait for before loading
   uint32_t *const *signal_peer = nullptr;   // [n_peers], with peer_rows > 0 (rows per peer a multiple of 32)
   const uint32_t *wait_counter = nullptr;

@@ -69,8 +69,8 @@ tp_reduce_bcast_kernel(const float4 *parts, int nparts, long long plane4, long l
                        PeerRows peers, int n_peers, long long dst4, const uint32_t *part_landed, uint32_t per_step,
                        const uint32_t *step, int *error, unsigned long long *trace) {
   if (blockIdx.x == 0 && threadIdx.x == 0) trace_store(trace, 0);
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) trace_store(trace, 1);
   __shared__ int ok;
   if (threadIdx.x == 0) {
@@ -123,8 +123,8 @@ tp_reduce_bcast_kernel(const float4 *parts, int nparts, long long plane4, long l
 __global__ void tp_step_end_kernel(const uint32_t *rows_landed, uint32_t per_step, uint32_t *step, uint32_t *xstep, int *error,
                                    unsigned long long *trace) {
   if (threadIdx.x == 0) trace_store(trace, 0);
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   if (threadIdx.x == 0) {
     trace_store(trace, 1);
     const uint32_t n = *reinterpret_cast<volatile uint32_t *>(step);
@@ -140,8 +140,8 @@ __global__ void tp_step_end_kernel(const uint32_t *rows_landed, uint32_t per_ste
 // the block into every other rank's input buffer over NVLink and counts the CTA in at every rank (itself included).
 __global__ void __launch_bounds__(256)
 tp_scatter_rows_kernel(const uint4 *src, long long n16, PeerCopy peers, int n_peers, int self) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n16; i += (long long)gridDim.x * blockDim.x) {
     const uint4 v = src[i];
     for (int d = 0; d < n_peers; ++d)
