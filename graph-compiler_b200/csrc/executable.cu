@@ -851,12 +851,15 @@ struct dnnl_graph_compiler_executable {
       const TensorSlot &wslot = plan.slots.at(st.in[1]);
       const bool w_const = wslot.where == TensorSlot::INPUT && p.tensors.at(st.in[1]).constant &&
                            in_stage[wslot.index].cached_host != nullptr;
-      if (!(w_const && comp_ready[size_t(st.scratch_slot)])) {
+      const bool zp = st.zp_a != 0;   // without a zero point there is nothing to take off
+      const bool sums = zp && !(w_const && comp_ready[size_t(st.scratch_slot)]);
+      if (sums) {
         colsum_s8(static_cast<const int8_t *>(addr(st.in[1])), comp, st.K, st.N, int32_t(st.zp_a), s);
         comp_ready[size_t(st.scratch_slot)] = w_const ? 1 : 0;
       }
       MatmulArgs m;
       m.A = addr(st.in[0]); m.B = addr(st.in[1]); m.M = st.M; m.N = st.N; m.K = st.K; m.int8 = 1;
+      m.early_inputs = sums;
       if (st.raw_acc) {
         // accumulators only: the raw s32 sums, then the zero-point term taken off per column
         m.out_kind = OUT_S32; m.out = addr(st.out[0]);
@@ -874,7 +877,7 @@ struct dnnl_graph_compiler_executable {
       }
       m.out_kind = OUT_DEQUANT_F32; m.out = addr(st.out[0]);
       m.scale = static_cast<const float *>(addr(st.in[2]));
-      m.comp = comp;
+      m.comp = zp ? comp : nullptr;
       m.bias_kind = st.has_bias ? BIAS_F32 : BIAS_NONE;
       m.bias = st.has_bias ? addr(st.in[3]) : nullptr;
       m.acc_dump = st.out.size() > 1 ? static_cast<int32_t *>(addr(st.out[1])) : nullptr;

@@ -102,8 +102,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // Everything above touched only shared and tensor memory and may overlap the tail of the kernel
   // ahead in the stream; from here on operands are read and results written.
   if (blockIdx.x == 0 && threadIdx.x == 0) trace_store(p.trace, 0);
-  pdl_wait();
-  pdl_launch_dependents();
+  // (operands that only the column-sum kernel ahead could delay are fetched at once; the results wait for it)
+  if (!p.early_inputs || (warp >= 2 && warp < 6)) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) trace_store(p.trace, 1);
 
   if (warp == 0 || warp == 6) {

@@ -82,6 +82,7 @@ struct GemmParams {
   const uint32_t *epoch;
   uint32_t wait_per_step;
   int *error;           // device int, set to an ErrCode on a bounded-wait time-out
+  int early_inputs;   // operands are complete when this kernel starts, whatever the kernel ahead still does
   unsigned long long *trace;   // optional time stamps of this launch (sm100_ptx.cuh: trace_store / trace_max)
   // TMA-store epilogue (one-CTA kernel, row-major orientation): tmC covers the output as
   // [planes][rows][cols] with a box of {128 bytes of columns, 32 rows, 1}; each epilogue warp hands its
