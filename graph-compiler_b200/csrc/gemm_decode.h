@@ -7,6 +7,7 @@
 namespace gcb {
 
 struct DecodeParams {
+  int kpb;        // K blocks of a stage
   int tiles;      // 128 output columns each
   int split;      // CTAs (a cluster) that share a tile's K range, every one with at least one K block
   uint32_t parts_bytes;   // shared memory for a CTA's partial sums: rows x 512 when split > 1

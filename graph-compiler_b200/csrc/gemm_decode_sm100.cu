@@ -5,9 +5,12 @@
 // (launch, set-up, the first loads' latency, the tail) and SMs without work because there are too few tiles, so
 //  * a tile's K range is shared by a cluster of 1 to 8 CTAs, which exchange their f32 partial sums through distributed
 //    shared memory: each finishes its share of the rows, adding the parts in K order.  No workspace, no second launch.
-//  * a CTA takes at most 107 KB of shared memory and 128 columns of tensor memory: two share an SM (up to 296 tiles run at
-//    once), and the next launch's CTAs move in beside this one's and have their set-up done - and, where the caller knows
-//    that nothing in flight writes the weights, their ring filled with weights - when this launch ends.
+//  * a CTA has an SM to itself and a ring of two-K-block stages (32 KB of weights and their activations; 192 KB under way
+//    with 16 rows): a stage's hand-shake takes 0.3 us whatever it holds, so one K block a stage held a CTA to 63 GB/s, and
+//    two CTAs to an SM made the SMs with two of them the last to finish.  Measured against that form: 16 x 28672 x 8192
+//    91 -> 76 us (6.2 TB/s), 64 x 28672 x 8192 118 -> 82, 32 x 4096 x 11008 24.8 -> 21, 16 x 1024 x 8192 14.3 -> 8.9 us.
+//  * where the caller knows that nothing in flight writes the weights, the ring is filled with them while the kernel ahead
+//    ends.
 // A variant that shared the K blocks of all tiles out evenly over the SMs (partial sums in global memory, finished by the
 // last warp to arrive) took 95 us instead of 14 at 32 x 4096 x 4096: one warp per tile cannot hide the latency of the sums.
 #include "gemm_decode.h"
@@ -21,8 +24,8 @@ namespace gcb {
 namespace {
 
 constexpr int kDecThreads = 224;
-constexpr int kDecMaxStages = 8;
-constexpr size_t kDecSmem = 109 * 1024;   // two CTAs per SM: 2 x (this + 1 KB reserved) within 228 KB
+constexpr int kDecMaxStages = 12;
+constexpr size_t kDecSmem = 226 * 1024;   // all but 1 KB of what a CTA may have
 
 struct DecBars {
   uint64_t full[kDecMaxStages], empty[kDecMaxStages], tmem_full[2], tmem_empty[2];
@@ -60,7 +63,7 @@ __device__ __forceinline__ void finish(const DecodeParams &p, uint32_t acc, int 
 }
 
 template <int KIND>
-__global__ void __launch_bounds__(kDecThreads, 2)
+__global__ void __launch_bounds__(kDecThreads, 1)
 gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ DecodeParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -72,7 +75,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stages = p.stages, kbs = p.k_blocks;
   const int split = p.split, rank = split > 1 ? int(cluster_ctarank()) : 0;
-  const int per = (kbs + split - 1) / split, kb0 = min(kbs, rank * per), kb1 = min(kbs, kb0 + per);   // this CTA's K blocks
+  const int kpb = p.kpb, per = ((kbs + split - 1) / split + kpb - 1) / kpb * kpb, kb0 = min(kbs, rank * per), kb1 = min(kbs, kb0 + per);   // this CTA's K blocks
   const int first = int(blockIdx.x) / split, stride = int(gridDim.x) / split;                         // its cluster's tiles
 
   if (threadIdx.x == 0) {
@@ -107,13 +110,15 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const CUtensorMap *tm = is_w ? &tmW : &tmX;
     const OperandGeom &g = is_w ? p.w : p.x;
     const uint32_t my_bytes = g.bytes, my_off = is_w ? 0u : p.w.bytes, boxes = g.boxes, box_bytes = g.box_bytes, box_mn = g.box_mn;
-    const bool mn = g.mn_major != 0, one = g.one_load != 0;
+    const bool mn = g.mn_major != 0, one = g.one_load != 0, k3d = g.k3d != 0;
     // Weights may be fetched before the kernel ahead has finished when nothing in flight writes them; everything else
     // (activations, results, and weights of unknown origin) waits for it.
     if (!(is_w && p.early_weights)) {
       if (is_w && elect_one()) {   // the first ring of weights at least comes to L2 meanwhile
-        for (int kb = kb0; kb < min(kb1, kb0 + stages); ++kb) {
-          if (!mn) tma_prefetch_2d(tm, kb * p.bk_elems, first * 128);
+        for (int kb = kb0; kb < min(kb1, kb0 + stages * kpb); kb += kpb) {
+          if (!mn && k3d) tma_prefetch_3d(tm, 0, first * 128, kb);
+          else if (!mn)
+            for (uint32_t i = 0; i < boxes; ++i) tma_prefetch_2d(tm, (kb + int(i)) * p.bk_elems, first * 128);
           else if (one) tma_prefetch_3d(tm, 0, kb * p.bk_elems, first * 128 / int(box_mn));
           else
             for (uint32_t i = 0; i < boxes; ++i) tma_prefetch_2d(tm, first * 128 + int(i * box_mn), kb * p.bk_elems);
@@ -129,7 +134,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     for (int t = first; t < p.tiles && !err; t += stride) {
       const int mn_off = is_w ? t * 128 : 0;
       const int grp = mn_off / int(box_mn ? box_mn : 1u);
-      for (int kb = kb0; kb < kb1; ++kb, ++issued) {
+      for (int kb = kb0; kb < kb1; kb += kpb, ++issued) {
         if (!behind && issued == uint32_t(stages)) {   // the ring is full: its first release is behind the kernel ahead
           pdl_wait();
           behind = true;
@@ -140,7 +145,9 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           const uint32_t dst = base + uint32_t(s) * stage_bytes + my_off;
           const int k_off = kb * p.bk_elems;
           mbar_expect_tx(full, my_bytes);
-          if (!mn) tma_load_2d(dst, tm, full, k_off, mn_off);
+          if (!mn && k3d) tma_load_3d(dst, tm, full, 0, mn_off, kb);
+          else if (!mn)
+            for (uint32_t i = 0; i < boxes; ++i) tma_load_2d(dst + i * box_bytes, tm, full, k_off + int(i) * p.bk_elems, mn_off);
           else if (one) tma_load_3d(dst, tm, full, 0, k_off, grp);
           else
             for (uint32_t i = 0; i < boxes; ++i) tma_load_2d(dst + i * box_bytes, tm, full, mn_off + int(i * box_mn), k_off);
@@ -163,6 +170,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     const uint64_t wd = umma_smem_desc(base, p.w.lbo, p.w.sbo), xd = umma_smem_desc(base + p.w.bytes, p.x.lbo, p.x.sbo);
     const uint32_t w_hi = uint32_t(wd >> 32), x_hi = uint32_t(xd >> 32), w_lo0 = uint32_t(wd), x_lo0 = uint32_t(xd);
     const uint32_t step = stage_bytes >> 4, w_k = p.w.kstep >> 4, x_k = p.x.kstep >> 4, idesc = p.idesc;
+    const uint32_t w_sub = p.w.sub_step >> 4, x_sub = p.x.sub_step >> 4;   // next K block of a stage
     auto desc = [](uint32_t lo, uint32_t hi) { return (uint64_t(hi) << 32) | uint64_t(lo); };
     int s = 0, err = 0;
     uint32_t ph = 0, seg = 0;
@@ -172,18 +180,21 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (!mbar_wait_warp(smem_u32(&bars->tmem_empty[acc]), acc_ph ^ 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
       tc_fence_after();
       const uint32_t d = tmem_base + acc * uint32_t(p.BN);
-      for (int kb = kb0; kb < kb1; ++kb) {
+      for (int kb = kb0; kb < kb1; kb += kpb) {
         if (!mbar_wait_warp(smem_u32(&bars->full[s]), ph)) { err = ERR_WAIT_FULL; break; }
         tc_fence_after();
-        const uint32_t wl = w_lo0 + uint32_t(s) * step, xl = x_lo0 + uint32_t(s) * step;
+        uint32_t wl = w_lo0 + uint32_t(s) * step, xl = x_lo0 + uint32_t(s) * step;
         if (elect_one()) {
+#pragma unroll 1
+          for (int i = 0; i < kpb; ++i, wl += w_sub, xl += x_sub) {
 #pragma unroll
-          for (uint32_t k = 0; k < 4; ++k) {
-            if (KIND == 0) umma_f16(d, desc(wl + k * w_k, w_hi), desc(xl + k * x_k, x_hi), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-            else           umma_i8(d, desc(wl + k * w_k, w_hi), desc(xl + k * x_k, x_hi), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            for (uint32_t k = 0; k < 4; ++k) {
+              if (KIND == 0) umma_f16(d, desc(wl + k * w_k, w_hi), desc(xl + k * x_k, x_hi), idesc, (kb + i > kb0 || k > 0) ? 1u : 0u);
+              else           umma_i8(d, desc(wl + k * w_k, w_hi), desc(xl + k * x_k, x_hi), idesc, (kb + i > kb0 || k > 0) ? 1u : 0u);
+            }
           }
           umma_commit(smem_u32(&bars->empty[s]));
-          if (kb + 1 == kb1) umma_commit(smem_u32(&bars->tmem_full[acc]));
+          if (kb + kpb >= kb1) umma_commit(smem_u32(&bars->tmem_full[acc]));
         }
         __syncwarp();
         if (++s == stages) { s = 0; ph ^= 1u; }
@@ -241,16 +252,24 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         break;
       }
       const uint32_t mine = smem_u32(parts + q * 32 + lane);
-      for (int orow = rank; orow < p.out_rows; orow += split) {
-        uint32_t w[8];
+      // four rows' parts are on their way at a time: fetched row by row, 32 rows took 4 us
+      for (int row0 = rank; row0 < p.out_rows; row0 += 4 * split) {
+        uint32_t w[4][8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c < split) w[c] = ld_shared_cluster(mapa_shared(mine + uint32_t(orow) * 512u, uint32_t(c)));
-        uint32_t sum = w[0];
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int c = 1; c < 8; ++c)
-          if (c < split) sum = KIND == 0 ? __float_as_uint(__fadd_rn(__uint_as_float(sum), __uint_as_float(w[c]))) : sum + w[c];
-        if (col_in) finish<KIND>(p, sum, orow, ocol, bias_bits, bias_f, scale_f, comp_i);
+          for (int c = 0; c < 8; ++c)
+            if (c < split && row0 + i * split < p.out_rows) w[i][c] = ld_shared_cluster(mapa_shared(mine + uint32_t(row0 + i * split) * 512u, uint32_t(c)));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int orow = row0 + i * split;
+          if (orow >= p.out_rows) break;
+          uint32_t sum = w[i][0];
+#pragma unroll
+          for (int c = 1; c < 8; ++c)
+            if (c < split) sum = KIND == 0 ? __float_as_uint(__fadd_rn(__uint_as_float(sum), __uint_as_float(w[i][c]))) : sum + w[i][c];
+          if (col_in) finish<KIND>(p, sum, orow, ocol, bias_bits, bias_f, scale_f, comp_i);
+        }
       }
       __syncwarp();
       if (lane < split) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->parts_out), uint32_t(lane)));

@@ -266,20 +266,21 @@ size_t matmul_scratch_bytes(int64_t M, int64_t N, int64_t K, int dtype_bytes, in
   return c.splits > 1 ? size_t(c.splits) * size_t(M) * size_t(N) * 4 : 0;
 }
 
-// CTAs that share a tile's K range.  A K block of a tile (16 KB of weights) takes a CTA 0.26 us when it is not held up by
-// the others, 6.2 TB/s bound them all, and a split costs about 1 us (partial sums exchanged in the cluster): the split with
-// the cheapest sum over the rounds, each CTA with four K blocks at least.  All measured at 32 x 11008 x 4096 and around it.
-static int decode_split(int tiles, int k_blocks, bool int8, int device, int *at_once) {
+// CTAs that share a tile's K range.  A K block of a tile (16 KB of weights) takes a CTA 0.17 us when it is not held up by
+// the others, the weights arrive at 7.5 TB/s at best, and handing parts round the cluster costs 1 us and 0.06 us for every row
+// that a CTA finishes: the split with the cheapest sum over the rounds.  Fitted to eighteen shapes from 300 x 1100 to
+// 28672 x 8192 with 1, 16, 32 and 64 rows, every split timed: 1.4 % behind the best one on average.
+static int decode_split(int tiles, int k_blocks, int kpb, int64_t rows, bool int8, int device, int *at_once) {
   int best = 1;
   double best_t = 1e30;
   for (int split = 1; split <= 8; ++split) {
-    if (split > 1 && k_blocks < 4 * split) break;
-    const int per = ceil_div(k_blocks, split);
+    const int per = ceil_div(ceil_div(k_blocks, split), kpb) * kpb;
     if (split > 1 && per * (split - 1) >= k_blocks) continue;   // the last CTA would have nothing to do
     const int clusters = decode_clusters_at_once(int8, device, split);
     if (clusters < 1) continue;
     const int rounds = ceil_div(tiles, clusters), active = std::min(tiles, clusters) * split;
-    const double t = rounds * per * std::max(0.26, active * 16384 / 6.2e6) + (split > 1 ? 1.0 + 0.1 * split : 0.0);
+    const double stream = double(tiles) * k_blocks * 16384 / 7.5e6;
+    const double t = std::max(stream, rounds * per * std::max(0.17, active * 16384 / 7.5e6)) + (split > 1 ? rounds * (1.0 + 0.06 * double(rows) / split) : 0.0);
     if (t < best_t) {
       best_t = t;
       best = split;
@@ -298,14 +299,15 @@ static void matmul_decode(const MatmulArgs &a, cudaStream_t stream) {
   p.k_blocks = ceil_div(a.K, p.bk_elems);
   p.tiles = ceil_div(a.N, 128);
   int clusters = 1;
-  p.split = decode_split(p.tiles, p.k_blocks, a.int8 != 0, dev.device, &clusters);
+  p.kpb = p.k_blocks >= 2 ? 2 : 1;
+  p.split = decode_split(p.tiles, p.k_blocks, p.kpb, a.M, a.int8 != 0, dev.device, &clusters);
   p.parts_bytes = p.split > 1 ? uint32_t(a.M) * 512u : 0u;
   p.BN = std::max(16, ceil_div(a.M, 16) * 16);
   p.early_weights = a.early_weights || a.early_inputs;
-  p.w = operand_geom(w_mn, 128, eb, 1);
-  p.x = operand_geom(x_mn, p.BN, eb, 1);
-  const CUtensorMap tmW = operand_tmap(p.w, a.int8 ? ElemType::S8 : ElemType::BF16, eb, a.B, a.N, a.K, 128, 1, a.ldb);
-  const CUtensorMap tmX = operand_tmap(p.x, a.int8 ? ElemType::U8 : ElemType::BF16, eb, a.A, a.M, a.K, p.BN, 1, a.lda);
+  p.w = operand_geom(w_mn, 128, eb, p.kpb);
+  p.x = operand_geom(x_mn, p.BN, eb, p.kpb);
+  const CUtensorMap tmW = operand_tmap(p.w, a.int8 ? ElemType::S8 : ElemType::BF16, eb, a.B, a.N, a.K, 128, p.kpb, a.ldb);
+  const CUtensorMap tmX = operand_tmap(p.x, a.int8 ? ElemType::U8 : ElemType::BF16, eb, a.A, a.M, a.K, p.BN, p.kpb, a.lda);
   p.idesc = umma_instr_desc(a.int8 ? 2u : 1u, 1u, a.int8 ? 0u : 1u, w_mn ? 1u : 0u, x_mn ? 1u : 0u, 128u, uint32_t(p.BN));
   p.tmem_cols = 32;
   while (p.tmem_cols < uint32_t(2 * p.BN)) p.tmem_cols <<= 1;

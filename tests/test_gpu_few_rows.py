@@ -87,3 +87,14 @@ torch.save([x.cpu() for x in o], sys.argv[1])
     for a, b in zip(*got):
         assert (a.float() - b.float()).abs().max() <= 3 * 2.0 ** -8 * b.float().abs().max()
         assert float((a == b).float().mean()) > 0.9
+
+
+@pytest.mark.parametrize("M,N,K,tb", [
+    (5, 640, 200, 1),       # rows that end inside a stage's second K block
+    (16, 300, 1096, 0),     # an odd number of K blocks, ragged columns
+    (64, 256, 4096, 0),     # two tiles: the widest cluster, eight rows for every CTA
+    (47, 512, 4224, 1),     # K blocks that no split divides evenly, rows that no split divides evenly
+    (3, 1024, 1984, 0),     # fewer rows than CTAs in the cluster
+])
+def test_few_rows_stages_of_two_k_blocks(M, N, K, tb):
+    test_few_rows_match_the_oracle_every_time(M, N, K, 0, tb)
