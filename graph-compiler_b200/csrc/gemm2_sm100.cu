@@ -23,6 +23,7 @@ constexpr int kStaging2 = 8192;   // per epilogue warp: two slabs of 32 rows x 1
 constexpr int kMaxStages2 = 8;
 
 struct PairBarriers {
+  uint4 table[4][kEpiTable / 16];   // per epilogue warp
   uint64_t full[kMaxStages2];
   uint64_t empty[kMaxStages2];
   uint64_t tmem_full[2];
@@ -209,6 +210,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
     uint8_t *stg = staging + (warp - 2) * kStaging2;
+    uint4 *table = bars->table[warp - 2];
     uint32_t tcount = 0;
     uint32_t slab = 0;   // TMA-store form: staging slab to fill next
     bool dead = false;
@@ -234,7 +236,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       tc_fence_after();
       const uint32_t t_addr = tmem_base + acc * uint32_t(p.BN) + (uint32_t(q * 32) << 16);
-      if (p.tma_store || p.row_store) gemm_epilogue_tile_tma<KIND>(p, t_addr, tm * 256 + int(rank) * 128, tn * p.BN, split, q, lane, stg, slab, cols);
+      if (p.tma_store || p.row_store) gemm_epilogue_tile_tma<KIND>(p, t_addr, tm * 256 + int(rank) * 128, tn * p.BN, split, q, lane, stg, slab, cols, table);
       else gemm_epilogue_tile<KIND, false>(p, t_addr, tm * 256 + int(rank) * 128, tn * p.BN, split, q, lane, stg);
       tc_fence_before();
       __syncwarp();

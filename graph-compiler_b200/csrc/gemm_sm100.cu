@@ -31,6 +31,7 @@ constexpr int kStageStaging = 8192;  // per epilogue warp: two slabs of 32 rows 
 constexpr int kMaxStages = 8;
 
 struct SmemBarriers {
+  uint4 table[4][kEpiTable / 16];   // per epilogue warp
   uint64_t full[kMaxStages];
   uint64_t empty[kMaxStages];
   uint64_t tmem_full[2];
@@ -240,6 +241,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
     uint8_t *stg = staging + (warp - 2) * kStageStaging;
+    uint4 *table = bars->table[warp - 2];
     uint32_t tcount = 0;
     uint32_t slab = 0;   // TMA-store form: staging slab to fill next
     bool dead = false;
@@ -268,7 +270,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const uint32_t t_addr = tmem_base + acc * uint32_t(p.BN) + (uint32_t(q * 32) << 16);
       const int nn0 = tn * p.BN;                 // first MMA column of the tile
 
-      if (!SWAPPED && (p.tma_store || p.row_store)) gemm_epilogue_tile_tma<KIND>(p, t_addr, tm * kBM, nn0, split, q, lane, stg, slab, cols);
+      if (!SWAPPED && (p.tma_store || p.row_store)) gemm_epilogue_tile_tma<KIND>(p, t_addr, tm * kBM, nn0, split, q, lane, stg, slab, cols, table);
       else gemm_epilogue_tile<KIND, SWAPPED>(p, t_addr, tm * kBM, nn0, split, q, lane, stg);
       tc_fence_before();
       __syncwarp();

@@ -22,6 +22,8 @@ enum ErrCode : int {
 
 // Geometry of one operand's pipeline stage in shared memory and of the
 // descriptors that walk it.
+constexpr int kEpiTable = 384;   // shared memory per epilogue warp for a slab's scale, bias and compensation
+
 struct OperandGeom {
   uint32_t mn_major;   // 0: K contiguous in memory, 1: MN contiguous
   uint32_t boxes;      // TMA boxes per stage

@@ -225,7 +225,7 @@ MatmulConfig model_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_byte
     const size_t km = size_t(c.bn) * 128;
     b_bytes = std::max(mn, km);
   }
-  const size_t budget = 232448 - 1024 - 4 * 8192 - 256;
+  const size_t budget = 232448 - 1024 - 4 * 8192 - 4 * kEpiTable - 256;
   const int kpb_eff = std::max(1, c.kpb);
   c.stages = int(std::min<size_t>(8, budget / ((a_bytes + b_bytes) * size_t(kpb_eff))));
   c.stages = std::max(2, std::min(c.stages, std::max(2, ceil_div(k_blocks, kpb_eff))));
@@ -585,7 +585,7 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   cudaError_t e;
   if (pair) {
     // stages are sized for the half B tile: recompute against the shared-memory budget
-    const size_t budget = 232448 - 1024 - 4 * 8192 - 256;
+    const size_t budget = 232448 - 1024 - 4 * 8192 - 4 * kEpiTable - 256;
     p.stages = int(std::max<size_t>(2, std::min<size_t>({size_t(8), budget / (p.a.bytes + p.b.bytes), size_t(std::max(2, p.k_blocks))})));
     if (a.force && a.force->stages >= 2) p.stages = std::min(p.stages, a.force->stages);
     const int grid = std::max(2, std::min(2 * units, dev.sm_count & ~1));
@@ -596,7 +596,7 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   } else {
     const int grid = std::max(1, std::min(units, cfg.grid > 0 ? cfg.grid : dev.sm_count));
     {
-      const size_t budget = 232448 - 1024 - 4 * 8192 - 256;
+      const size_t budget = 232448 - 1024 - 4 * 8192 - 4 * kEpiTable - 256;
       const int fit = int(budget / (p.a.bytes + p.b.bytes));
       if (fit < 2) throw std::invalid_argument("matmul stage does not fit twice in shared memory");
       p.stages = std::max(2, std::min({p.stages, fit, std::max(2, ceil_div(p.k_blocks, kpb))}));
