@@ -237,6 +237,15 @@ MatmulConfig model_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_byte
   // 512 x 4096 x 16384 split in two: 64.3 against 68.6 us), slower on large square shapes (4096^3: 109.5 against 103.1 us).
   c.pair = (!c.swapped && dtype_bytes == 2 && c.bn == 256 && c.kpb <= 1 && M % 256 == 0 && M <= 1024 && N >= 2048 && N % 256 == 0 &&
             k_blocks / std::max(1, c.splits) >= 16) ? 1 : 0;
+  // ... and, with the MMAs issued from uniform registers, on larger unsplit shapes too (half the weight bytes per SM, which
+  // under the power cap is also clock): 16384^3 7.38 -> 6.65 ms, 8192^3 877 -> 843 us, 4096^3 116 -> 109, 2048 x 4096 x 16384
+  // 235 -> 215, 5000 x 20000 x 2000 439 -> 407, 4096 x 1024 x 4096 34 -> 30, 8192 x 512 x 2048 21.5 -> 19.7, 2048^3 18.9 -> 18.4.
+  // Below sixteen K blocks a tile is too short to hide the hand-offs (8192 x 4096 x 512: 38 against 43 us).
+  if (!c.swapped && dtype_bytes == 2 && c.bn == 256 && c.kpb <= 1 && c.splits == 1 && max_splits > 1 && M >= 1024 && k_blocks >= 16 &&
+      ceil_div(2 * ceil_div(M, 256) * ceil_div(N, 256), sm_count & ~1) <= ceil_div(tiles, sm_count)) {   // rows padded to 256 cost no wave
+    c.pair = 1;
+    c.group_m = 8;   // 16384^3: 6.65 ms against 6.79 with four, whose reason (above) is the one-CTA tile
+  }
   // u8 x s8 on several waves of tiles: pairs measured 8192^3 393.5 against 418.6 us, 4096^3 68.5 against 70.5 us
   // (1024 x 4096 x 4096, a single wave: 31.7 against 31.9 us - left on one CTA per tile)
   if (!c.swapped && dtype_bytes == 1 && c.bn == 256 && c.kpb <= 1 && c.splits == 1 && M % 256 == 0 && N % 256 == 0 &&
