@@ -28,6 +28,7 @@
 // 128 columns each = 512 columns.
 #include "attention.h"
 
+#include <algorithm>
 #include <cmath>
 #include <stdexcept>
 
@@ -51,6 +52,7 @@ struct AttParams {
   void *O;
   int *error;
   int q_pairs;         // ceil(seq / 256)
+  int group;           // causal: (batch, head) units whose query pairs are worked off together
 };
 
 struct AttBars {
@@ -113,9 +115,15 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   AttBars *bars = reinterpret_cast<AttBars *>(smem + (2 + kRing + 2) * kSlot);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heavier (later) query pairs first when causal
-  const int pair = p.causal ? (p.q_pairs - 1 - int(blockIdx.x)) : int(blockIdx.x);
-  const int bh = blockIdx.y;
+  int pair = int(blockIdx.x), bh = int(blockIdx.y);
+  if (p.causal) {
+    // Heavier (later) query pairs first, over all units of a group: unit by unit, the heavy pairs of the last units started
+    // when the SMs had little else left (2 x 32 x 3001: 188 -> 176 us, 1 x 32 x 2048 62 -> 51, 1 x 16 x 8192 298 -> 264).
+    const unsigned per_group = unsigned(p.group) * unsigned(p.q_pairs), at = blockIdx.y * gridDim.x + blockIdx.x;
+    const unsigned g = at / per_group, r = at - g * per_group, units = min(unsigned(p.group), unsigned(p.bh) - g * unsigned(p.group));
+    pair = p.q_pairs - 1 - int(r / units);
+    bh = int(g * unsigned(p.group) + r % units);
+  }
   const int q_base0 = pair * 256, q_base1 = q_base0 + 128;
   const bool act1 = q_base1 < p.seq;
   const int kv_tiles_all = (p.seq + kTile - 1) / kTile;
@@ -185,16 +193,16 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    // The whole warp walks the tiles, one elected lane issues (see elect_one).
-    {
+    if (lane == 0) {
       const uint32_t idesc_qk = umma_instr_desc(1, 1, 1, 0, 0, 128, 128);   // A, B K-major
       // A (P) and B (V) must have the same 16-bit format: kind::f16 with an f16 A and a bf16 B operand
       // raises an illegal-instruction fault on sm_100a, so P is rounded to bf16 like V
       const uint32_t idesc_pv = umma_instr_desc(1, 1, 1, 0, 1, 128, 128);   // B (V) MN-major
       const int nt[2] = {n0, n1};
       int err = 0;
-      // Descriptors are split into a constant high word and a low word (start address in 16-byte units |
-      // leading offset << 16) that advances by a compile-time constant per K step.
+      // This thread's instruction stream is the tensor pipe's critical path: descriptors are split into
+      // a constant high word and a low word (start address in 16-byte units | leading offset << 16)
+      // that advances by a compile-time constant per K step.
       const uint32_t hi_k = uint32_t(umma_smem_desc(0, 16, 1024) >> 32);
       const uint32_t hi_v = uint32_t(umma_smem_desc(0, 16384, 1024) >> 32);
       auto lo_k = [](uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); };
@@ -209,25 +217,22 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       auto issue_qk = [&](int t, uint32_t kslot) {
         const uint32_t d = tmem + uint32_t(t) * 128u;
         const uint32_t a = q_lo[t], b = lo_k(kslot);
-        if (elect_one()) {
 #pragma unroll
-          for (int s = 0; s < 8; ++s) {
-            const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
-            umma_f16(d, dsc(a + off, hi_k), dsc(b + off, hi_k), idesc_qk, s > 0 ? 1u : 0u);
-          }
-          umma_commit(s_full_b[t]);
+        for (int s = 0; s < 8; ++s) {
+          const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
+          umma_f16(d, dsc(a + off, hi_k), dsc(b + off, hi_k), idesc_qk, s > 0 ? 1u : 0u);
         }
-        __syncwarp();
+        umma_commit(s_full_b[t]);
       };
       // ring position of the next entry to consume (same order as the producer fills it)
       int slot = 0;
       uint32_t ph = 0;
-      auto ring_wait = [&]() { return mbar_wait_warp(smem_u32(&bars->kv_full[slot]), ph); };
+      auto ring_wait = [&]() { return mbar_wait(smem_u32(&bars->kv_full[slot]), ph); };
       auto ring_release = [&]() {
-        if (elect_one()) umma_commit(smem_u32(&bars->kv_empty[slot]));   // free once the MMAs issued so far retire
+        umma_commit(smem_u32(&bars->kv_empty[slot]));   // free once the MMAs issued so far retire
         if (++slot == kRing) { slot = 0; ph ^= 1u; }
       };
-      if (!mbar_wait_warp(smem_u32(&bars->q_full), 0)) err = ERR_WAIT_FULL;
+      if (!mbar_wait(smem_u32(&bars->q_full), 0)) err = ERR_WAIT_FULL;
       if (!err && !ring_wait()) err = ERR_WAIT_FULL;
       if (!err) {
         tc_fence_after();
@@ -242,7 +247,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const uint32_t kslot = ring_s + uint32_t(slot) * kSlot;
           for (int t = 0; t < 2 && !err; ++t) {
             if (j + 1 >= nt[t]) continue;
-            if (!mbar_wait_warp(s_free_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
+            if (!mbar_wait(s_free_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
             tc_fence_after();
             issue_qk(t, kslot);
           }
@@ -254,24 +259,21 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t v_lo = lo_v(ring_s + uint32_t(slot) * kSlot);
         for (int t = 0; t < 2 && !err; ++t) {
           if (j >= nt[t]) continue;
-          if (!mbar_wait_warp(p_ready_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
+          if (!mbar_wait(p_ready_b[t], uint32_t(j) & 1u)) { err = ERR_WAIT_TMEM_EMPTY; break; }
           tc_fence_after();
           const uint32_t d = tmem + 256u + uint32_t(t) * 128u;
           const uint32_t a = p_lo[t];
-          if (elect_one()) {
 #pragma unroll
-            for (int s = 0; s < 8; ++s) {
-              const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
-              umma_f16(d, dsc(a + off, hi_k), dsc(v_lo + uint32_t(s) * 128u, hi_v), idesc_pv, (j > 0 || s > 0) ? 1u : 0u);
-            }
-            umma_commit(pv_full_b[t]);
+          for (int s = 0; s < 8; ++s) {
+            const uint32_t off = uint32_t(s >> 2) * 1024u + uint32_t(s & 3) * 2u;
+            umma_f16(d, dsc(a + off, hi_k), dsc(v_lo + uint32_t(s) * 128u, hi_v), idesc_pv, (j > 0 || s > 0) ? 1u : 0u);
           }
-          __syncwarp();
+          umma_commit(pv_full_b[t]);
         }
         if (err) break;
         ring_release();
       }
-      if (err && lane == 0) atomicExch(p.error, err);
+      if (err) atomicExch(p.error, err);
     }
   } else {
     // ---------------------------------------------------------------- softmax / epilogue
@@ -470,6 +472,10 @@ void attention_bf16(const void *Q, const void *K, const void *V, void *O, int64_
   p.O = O;
   p.error = dev.d_error;
   p.q_pairs = int((seq + 255) / 256);
+  // as many units as keep their keys and values in half the L2 cache (more would read them from HBM for every query pair)
+  const int64_t fit = std::max<int64_t>(1, (int64_t(64) << 20) / (4 * seq * dim)), groups = (bh + fit - 1) / fit;
+  // and unit by unit when all pairs run at once (4 x 2048: 34 against 35 us)
+  p.group = int64_t(p.q_pairs) * bh <= dev.sm_count ? 1 : int((bh + groups - 1) / groups);
   const size_t smem = 1024 + size_t(2 + kRing + 2) * kSlot + sizeof(AttBars);
   static bool configured[64] = {};
   if (!configured[dev.device & 63]) {
