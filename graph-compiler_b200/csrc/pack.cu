@@ -94,6 +94,9 @@ void matmul_bf16_packed(const MatmulArgs &a, void *pack, cudaStream_t stream) {
   Operand o[2];
   operands(a, o);
   MatmulArgs m = a;
+  // pack_rows lets the matmul start while it still writes: a packed operand is not complete until its wait is over
+  m.early_inputs = 0;
+  if (o[1].pack) m.early_weights = 0;
   uint8_t *at = static_cast<uint8_t *>(pack);
   for (int i = 0; i < 2; ++i) {
     if (!o[i].pack) continue;

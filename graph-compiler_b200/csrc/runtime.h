@@ -117,7 +117,8 @@ struct MatmulArgs {
                                 // (plane = peer_plane * peer_splits + split; the owner's buffer holds n_peers * peer_splits planes)
   void *const *peer_out = nullptr;
   int peer_multicast = 0;       // 1: n_peers == 1 and peer_out[0] is an NVLink multicast address of all ranks' buffers
-  int early_weights = 0;        // few-rows form: no work in flight on the device writes B (see gemm_decode_sm100.cu)
+  int early_weights = 0;        // few-rows form: no work in flight on the device writes B (see gemm_decode_sm100.cu); a
+                                // statement about the caller's B, not about a packed copy of it
   int early_inputs = 0;         // the kernel ahead in the stream is colsum_s8: A and B are complete, comp is not yet
   int plain_stores = 0;         // 1: `out` is written with ordinary stores (memory of the host)
   const MatmulConfig *force = nullptr; // optional override
