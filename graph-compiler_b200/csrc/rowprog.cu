@@ -275,16 +275,18 @@ struct Compiler {
     g.prog.op[g.prog.n++] = o;
     return true;
   }
-  // The matmul step whose K-split planes may be summed here: a bf16 result that only this run reads.
+  // The matmul step whose K-split planes may be summed here: a bf16 result that only this run reads (its own memory is
+  // then never written, so no step before or after the run may look there).
   int deferrable(size_t id) const {
     if (leaves(id)) return -1;
+    int producer = -1;
     for (int k = 0; k < first; ++k) {
       const Step &st = step(k);
       if (std::find(st.in.begin(), st.in.end(), id) != st.in.end()) return -1;
       if (st.out.size() == 1 && st.out[0] == id)
-        return st.kind == StepKind::MATMUL && !st.has_bias && !st.relu && tensor(id).dtype == DType::BF16 ? k : -1;
+        producer = st.kind == StepKind::MATMUL && !st.has_bias && !st.relu && tensor(id).dtype == DType::BF16 ? k : -1;
     }
-    return -1;
+    return producer;
   }
   bool load(size_t id) {   // brings an operand into a register
     if (reg.count(id)) return true;

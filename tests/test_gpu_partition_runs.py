@@ -1,4 +1,6 @@
 """Partitions whose steps hand buffers on to each other inside one call: packed weights, deferred partial sums."""
+import json
+
 import pytest
 import torch
 
@@ -40,3 +42,40 @@ def test_packed_weights_of_a_chain_of_few_rows(batch, hidden):
         torch.cuda.synchronize()
         assert lib.device_error() == 0
         assert torch.equal(out, want[turn & 1]), f"turn {turn}"
+
+
+def _tensor(tid, *shape):
+    return {"id": tid, "dtype": "bf16", "shape": list(shape)}
+
+
+def _partition(ops, inputs, outputs):
+    graph = [{"kind": kind, "inputs": ins, "outputs": [out]} for kind, ins, out in ops]
+    return json.dumps({"version": "3.5.0", "engine_kind": "cpu", "fpmath_mode": "any", "input_ports": inputs, "output_ports": outputs, "graph": graph})
+
+
+M, N, K = 128, 1024, 4096   # few tiles and a long K: the selector splits K, so a run may add the partial sums itself
+
+
+@pytest.mark.parametrize("reader", ["matmul", "earlier run"])
+def test_a_split_result_with_a_second_reader_is_written(reader):
+    """y = x w1 with its K split; a run of elementwise steps adds y to z, and z (or what z is made of) needs y as well."""
+    assert lib.select_matmul_config(M, N, K).splits > 1
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, w1, w2, s = _bf(g, M, K), _bf(g, K, N, k=K ** -0.5), _bf(g, N, N, k=N ** -0.5), _bf(g, N)
+    t = {i: _tensor(i, M, N) for i in range(10, 16)}
+    ops = [("MatMul", [_tensor(0, M, K), _tensor(1, K, N)], t[10])]
+    z_in = 10
+    if reader == "earlier run":
+        ops += [("Multiply", [t[10], _tensor(3, N)], t[11]), ("ReLU", [t[11]], t[12])]
+        z_in = 12
+    ops += [("MatMul", [t[z_in], _tensor(2, N, N)], t[13]), ("Add", [t[10], t[13]], t[14]), ("Multiply", [t[14], _tensor(3, N)], t[15])]
+    exe = api.GraphCompiler().compile(_partition(ops, [0, 1, 2, 3], [15]))
+    y = lib.matmul_bf16(x, w1)
+    z = lib.matmul_bf16(torch.relu(y * s) if reader == "earlier run" else y, w2)
+    want = (y + z) * s
+    for _ in range(3):
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        exe.execute_on_stream({0: x, 1: w1, 2: w2, 3: s}, {15: out})
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    assert lib.device_error() == 0
