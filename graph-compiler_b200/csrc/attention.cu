@@ -52,7 +52,7 @@ struct AttParams {
   void *O;
   int *error;
   int q_pairs;         // ceil(seq / 256)
-  int group;           // causal: (batch, head) units whose query pairs are worked off together
+  int group;           // causal: (batch, head) units whose query pairs are worked off together; 1: unit by unit
 };
 
 struct AttBars {
@@ -115,15 +115,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   AttBars *bars = reinterpret_cast<AttBars *>(smem + (2 + kRing + 2) * kSlot);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int pair = int(blockIdx.x), bh = int(blockIdx.y);
-  if (p.causal) {
-    // Heavier (later) query pairs first, over all units of a group: unit by unit, the heavy pairs of the last units started
-    // when the SMs had little else left (2 x 32 x 3001: 188 -> 176 us, 1 x 32 x 2048 62 -> 51, 1 x 16 x 8192 298 -> 264).
-    const unsigned per_group = unsigned(p.group) * unsigned(p.q_pairs), at = blockIdx.y * gridDim.x + blockIdx.x;
-    const unsigned g = at / per_group, r = at - g * per_group, units = min(unsigned(p.group), unsigned(p.bh) - g * unsigned(p.group));
-    pair = p.q_pairs - 1 - int(r / units);
-    bh = int(g * unsigned(p.group) + r % units);
-  }
+  // The grid is [groups of units][query pairs][units of a group].  Causal: heavier (later) query pairs first, over all units
+  // of a group; unit by unit, the heavy pairs of the last units started when the SMs had little else left (2 x 32 x 3001:
+  // 188 -> 176 us, 1 x 32 x 2048 62 -> 51, 1 x 16 x 8192 298 -> 264).
+  const int pair = p.causal ? p.q_pairs - 1 - int(blockIdx.y) : int(blockIdx.y), bh = int(blockIdx.z) * p.group + int(blockIdx.x);
+  if (bh >= p.bh) return;   // the last group may have fewer units
   const int q_base0 = pair * 256, q_base1 = q_base0 + 128;
   const bool act1 = q_base1 < p.seq;
   const int kv_tiles_all = (p.seq + kTile - 1) / kTile;
@@ -472,17 +468,22 @@ void attention_bf16(const void *Q, const void *K, const void *V, void *O, int64_
   p.O = O;
   p.error = dev.d_error;
   p.q_pairs = int((seq + 255) / 256);
-  // as many units as keep their keys and values in half the L2 cache (more would read them from HBM for every query pair)
-  const int64_t fit = std::max<int64_t>(1, (int64_t(64) << 20) / (4 * seq * dim)), groups = (bh + fit - 1) / fit;
-  // and unit by unit when all pairs run at once (4 x 2048: 34 against 35 us)
-  p.group = int64_t(p.q_pairs) * bh <= dev.sm_count ? 1 : int((bh + groups - 1) / groups);
+  // Groups of about two and a half waves of query pairs, no more units in one than keep their keys and values in half the L2
+  // cache (beyond it they would come from HBM for every pair).  All units in one group lost what neighbouring pairs share in
+  // L2 where there are many short ones: 244 x 1062 140.9 us, in groups 137, unit by unit 135.5; 99 x 2959 268 / 266 / 280;
+  // 30 x 5074 207 / 204 / 229.  Unit by unit when all pairs run at once (10 x 3436: 51.3 against 51.7 us, nothing to gain) and
+  // when only two pairs, hardly unlike, meet many waves (888 x 328: 108.6 against 110.6 us; at four waves 51.2 against 47.3).
+  const int64_t pairs = int64_t(p.q_pairs) * bh, sms = dev.sm_count;
+  const int64_t fit = std::max<int64_t>(1, (int64_t(64) << 20) / (4 * seq * dim));
+  const int64_t groups = std::max({int64_t(1), (bh + fit - 1) / fit, (4 * pairs + 5 * sms) / (10 * sms)});
+  p.group = !causal || pairs <= sms || (p.q_pairs <= 2 && pairs > 10 * sms) ? 1 : int((bh + groups - 1) / groups);
   const size_t smem = 1024 + size_t(2 + kRing + 2) * kSlot + sizeof(AttBars);
   static bool configured[64] = {};
   if (!configured[dev.device & 63]) {
     GCB_CUDA(cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     configured[dev.device & 63] = true;
   }
-  dim3 grid(unsigned(p.q_pairs), unsigned(bh));
+  dim3 grid(unsigned(p.group), unsigned(p.q_pairs), unsigned((bh + p.group - 1) / p.group));
   attention_kernel<<<grid, kAttThreads, smem, stream>>>(tq, tk, tv, p);
   GCB_CUDA(cudaGetLastError());
   count_launch();

@@ -53,6 +53,25 @@ def test_attention_small(bh, S, causal):
     print(f"attention bh={bh} S={S} causal={causal}: max_abs={mx:.4g} within_plain_1e-2={plain:.5f} rounding_term_used={used:.3f}")
 
 
+@pytest.mark.parametrize("bh,S", [
+    (399, 300),    # several groups of units, the last one not full
+    (760, 257),    # two pairs and many waves: unit by unit
+    (74, 520),     # a little more than one wave of query pairs: one group
+    (149, 100),    # one pair per unit
+])
+def test_causal_units_in_any_order(bh, S):
+    """Causal query pairs are worked off over groups of units: every unit has the bits that it has alone."""
+    g = torch.Generator(device="cuda").manual_seed(bh)
+    Q, K, V = (torch.randn(bh, S, 128, generator=g, device="cuda").bfloat16() for _ in range(3))
+    O = torch.full_like(Q, float("nan"))
+    lib.attention_bf16(Q, K, V, 1.0 / math.sqrt(128), True, out=O)
+    alone = torch.cat([lib.attention_bf16(Q[i:i + 1], K[i:i + 1], V[i:i + 1], 1.0 / math.sqrt(128), True) for i in range(bh)])
+    torch.cuda.synchronize()
+    assert lib.device_error() == 0
+    assert torch.equal(O, alone)
+    _check(O[-1], Q[-1], K[-1], V[-1], 1.0 / math.sqrt(128), True, f"last of {bh} x {S}")
+
+
 @pytest.mark.parametrize("causal", [False, True])
 def test_attention_full_size_units(causal):
     """BASELINE configs[3]: batch 16, 32 heads, seq 2048, head_dim 128 through the SDPA partition;
