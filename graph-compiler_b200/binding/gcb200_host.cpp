@@ -18,7 +18,7 @@ namespace {
 
 // interned names and cached objects of the torch module (set by setup())
 PyObject *s_data_ptr, *s_shape, *s_is_cuda, *s_dtype, *s_is_contiguous;
-PyObject *t_tensor, *t_bf16, *f_get_device, *f_raw_stream;
+PyObject *t_tensor, *t_bf16, *f_get_device, *f_raw_stream, *t_ndarray;
 
 struct Ref {   // owned reference
   PyObject *p;
@@ -128,19 +128,30 @@ struct Pack {
   dnnl_graph_compiler_tensor t[kMaxTensors + 1];
   int64_t dims[kMaxTensors][DNNL_MAX_NDIMS];
   Py_buffer views[kMaxTensors];
-  int n = 0, n_views = 0;
+  PyObject *held[kMaxTensors];   // the call runs without the interpreter's lock: another thread may change the dictionary
+  int n = 0, n_views = 0, n_held = 0;
   ~Pack() {
     for (int i = 0; i < n_views; ++i) PyBuffer_Release(&views[i]);
+    for (int i = 0; i < n_held; ++i) Py_DECREF(held[i]);
   }
-  // 1: packed, 0: something this path does not take (the caller packs it in Python), -1: error
+  // 1: packed, 0: something this path does not take (the caller packs it in Python), -1: error.  Only tensors and numpy
+  // arrays are taken: other objects with a buffer (bytes, memoryview) are no arguments of a partition, and an output among
+  // them could be memory that must not change.
   int add(PyObject *key, PyObject *val) {
     if (n == kMaxTensors) return 0;
+    const bool tensor = PyObject_TypeCheck(val, reinterpret_cast<PyTypeObject *>(t_tensor));
+    if (!tensor && !(t_ndarray && PyObject_TypeCheck(val, reinterpret_cast<PyTypeObject *>(t_ndarray)))) return 0;
     const size_t id = PyLong_AsSize_t(key);
-    if (id == size_t(-1) && PyErr_Occurred()) return -1;
+    if (id == size_t(-1) && PyErr_Occurred()) {
+      PyErr_Clear();
+      return 0;
+    }
+    Py_INCREF(val);
+    held[n_held++] = val;
     int64_t *d = dims[n];
     void *p;
     int nd;
-    if (PyObject_TypeCheck(val, reinterpret_cast<PyTypeObject *>(t_tensor))) {
+    if (tensor) {
       nd = shape(val, d, DNNL_MAX_NDIMS);
       if (nd == -2) return 0;
       if (nd < 0 || !address(val, &p)) return -1;
@@ -202,11 +213,11 @@ PyObject *execute(PyObject *, PyObject *const *a, Py_ssize_t n) {
   return PyLong_FromLong(st);
 }
 
-// setup(torch.Tensor, torch.bfloat16, get_device, get_raw_stream)
+// setup(torch.Tensor, torch.bfloat16, get_device, get_raw_stream, numpy.ndarray)
 PyObject *setup(PyObject *, PyObject *const *a, Py_ssize_t n) {
-  if (n != 4) return PyErr_Format(PyExc_TypeError, "setup takes 4 arguments"), nullptr;
-  PyObject **slots[4] = {&t_tensor, &t_bf16, &f_get_device, &f_raw_stream};
-  for (int i = 0; i < 4; ++i) {
+  if (n != 5) return PyErr_Format(PyExc_TypeError, "setup takes 5 arguments"), nullptr;
+  PyObject **slots[5] = {&t_tensor, &t_bf16, &f_get_device, &f_raw_stream, &t_ndarray};
+  for (int i = 0; i < 5; ++i) {
     Py_INCREF(a[i]);
     Py_XSETREF(*slots[i], a[i]);
   }

@@ -113,6 +113,11 @@ _host = None         # the compiled module, once torch is there to be bound
 _host_module = None
 
 
+def _ndarray():
+    numpy = sys.modules.get("numpy")   # a program that holds arrays has imported it
+    return numpy.ndarray if numpy is not None else type(None)
+
+
 def host():
     """The compiled call path of the small, repeated calls (binding/gcb200_host.cpp)."""
     global _host, _host_module
@@ -128,11 +133,12 @@ def host():
         loader = importlib.machinery.ExtensionFileLoader("_gcb200_host", HOST_PATH)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_gcb200_host", loader))
         loader.exec_module(mod)
-        mod.setup(type(None), None, None, None)
+        mod.setup(type(None), None, None, None, _ndarray())
         _host_module = mod
     torch = sys.modules.get("torch")   # a program that holds tensors has imported it
     if torch is not None:
-        _host_module.setup(torch.Tensor, torch.bfloat16, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream)
+        _host_module.setup(torch.Tensor, torch.bfloat16, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream,
+                           _ndarray())
         _host = _host_module
     return _host_module
 

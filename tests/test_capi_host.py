@@ -282,6 +282,36 @@ def test_tile_selection_for_the_benchmark_shapes():
         assert 16 <= c.bn <= 256 and c.bn % 16 == 0 and 2 <= c.stages <= 8 and c.splits >= 1 and c.grid >= 1
 
 
+class _Lent:
+    """An object with a buffer and a shape that is neither a tensor nor an array."""
+    shape = (8, 8)
+
+    def __buffer__(self, flags):
+        return memoryview(bytearray(64)).cast("B", (8, 8))
+
+
+@pytest.mark.parametrize("where", ["input", "output"])
+@pytest.mark.parametrize("make", [lambda: bytes(8 * 16 * 4), lambda: bytearray(8 * 8 * 4), lambda: memoryview(bytearray(64)).cast("B", (8, 8)), _Lent],
+                         ids=["bytes", "bytearray", "memoryview", "lent"])
+def test_arguments_that_are_no_tensors_are_refused(where, make):
+    """Whatever merely lends its bytes is no argument: an output among them could be an immutable object, and their shape
+    counts bytes where a tensor's counts elements."""
+    import numpy as np
+
+    js, ids, out = partitions.mlp(8, (16, 8), dtype="f32")
+    exe = api.GraphCompiler().compile(js)
+    ins = {0: np.zeros((8, 16), np.float32), 1: np.zeros((16, 8), np.float32), 2: np.zeros(8, np.float32)}
+    outs = {out: np.zeros((8, 8), np.float32)}
+    (ins if where == "input" else outs)[0 if where == "input" else out] = make()
+    class Stream:
+        cuda_stream = 0
+
+    with pytest.raises(AttributeError):   # refused before the library sees it
+        exe.execute(ins, outs)
+    with pytest.raises(AttributeError):
+        exe.execute_on_stream(ins, outs, Stream())
+
+
 def test_launchers_fail_loudly_without_a_device():
     import torch
 
