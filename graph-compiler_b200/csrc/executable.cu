@@ -768,7 +768,7 @@ struct dnnl_graph_compiler_executable {
     return small_out_host.ptr && b >= small_out_host.ptr && b < small_out_host.ptr + small_out_host.bytes;
   }
 
-  // Steps [begin, end) in order, elementwise runs as one kernel where their tensors are 16-byte aligned.
+  // Steps [begin, end) in order, elementwise runs as one kernel where their tensors allow it.
   template <class Addr>
   void run_steps(size_t begin, size_t end, Addr &addr, const std::vector<void *> &in_ptr, cudaStream_t s) const {
     // Whether this call has launched something: every kernel of this library lets the next one start only behind its own
@@ -780,12 +780,11 @@ struct dnnl_graph_compiler_executable {
       if (group_at[k] >= 0) {
         const RowGroup &g = groups[size_t(group_at[k])];
         RowProgram p = g.prog;
-        bool ok = size_t(g.last) < end;
         for (size_t i = 0; i < g.ids.size(); ++i) {
           p.ptr[i] = addr(g.ids[i]);
           p.planes[i] = 0;
-          ok &= (reinterpret_cast<uintptr_t>(p.ptr[i]) & 15) == 0;
         }
+        const bool ok = size_t(g.last) < end && row_program_fits(g, p.ptr);
         for (int m : g.deferred) {
           const Step &ms = plan.steps[size_t(m)];
           if (planes[size_t(m)] == 0) continue;

@@ -268,6 +268,9 @@ struct Compiler {
     if (it != slot.end()) return it->second;
     if (g.ids.size() == size_t(kProgPtrs)) return -1;
     g.ids.push_back(id);
+    g.bytes.push_back(plan.slots.at(id).bytes);
+    g.stored.push_back(0);
+    g.whole.push_back(form(tensor(id)) == Form::FULL);
     return slot[id] = uint8_t(g.ids.size() - 1);
   }
   bool emit(const RowOp &o) {
@@ -395,6 +398,7 @@ struct Compiler {
         const int p = pointer(st.out[0]);
         if (p < 0) return false;
         w.ptr = uint8_t(p);
+        g.stored[size_t(p)] = 1;
         stored.push_back(st.out[0]);
         if (!emit(w)) return false;
       }
@@ -411,6 +415,19 @@ struct Compiler {
 };
 
 } // namespace
+
+bool row_program_fits(const RowGroup &g, void *const *ptr) {
+  auto at = [&](size_t i) { return reinterpret_cast<uintptr_t>(ptr[i]); };
+  for (size_t i = 0; i < g.ids.size(); ++i) {
+    if (at(i) & 15) return false;
+    if (!g.stored[i]) continue;
+    for (size_t k = 0; k < g.ids.size(); ++k) {
+      if (k == i || at(i) >= at(k) + g.bytes[k] || at(k) >= at(i) + g.bytes[i]) continue;
+      if (!(at(i) == at(k) && g.whole[i] && g.whole[k] && g.bytes[i] == g.bytes[k])) return false;
+    }
+  }
+  return true;
+}
 
 std::vector<RowGroup> plan_row_groups(const Plan &plan) {
   std::vector<RowGroup> groups;

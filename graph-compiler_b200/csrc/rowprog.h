@@ -41,13 +41,20 @@ struct RowGroup {
   int first = 0, last = 0;
   RowProgram prog;
   std::vector<size_t> ids;     // tensor behind each pointer slot
+  std::vector<size_t> bytes;   // its size
+  std::vector<char> stored, whole;   // the program writes it; it has the run's shape (a thread touches its own elements only)
   std::vector<int> deferred;   // matmul steps whose K-split planes the program may sum itself (their result has no other reader)
 };
 
 // Runs worth fusing (two steps or more).  Host logic; steps that do not fit are left out.
 std::vector<RowGroup> plan_row_groups(const Plan &plan);
 
-// All pointers must be 16-byte aligned (the caller runs the steps one by one otherwise).
+// Whether the tensors lie where the program may run on them: 16-byte aligned, and nothing is stored over memory that
+// another thread has still to load - a caller may hand in buffers that overlap, and one after the other the steps allow it.
+// The one overlap that is fine is a result in the place of an operand of the same shape and element size.
+bool row_program_fits(const RowGroup &g, void *const *ptr);
+
+// The caller runs the steps one by one where row_program_fits says no.
 void launch_row_program(const RowProgram &p, cudaStream_t stream);
 
 } // namespace gcb

@@ -79,3 +79,48 @@ def test_a_split_result_with_a_second_reader_is_written(reader):
         torch.cuda.synchronize()
         assert torch.equal(out, want)
     assert lib.device_error() == 0
+
+
+def _floats(tid, *shape):
+    return dict(_tensor(tid, *shape), dtype="f32")
+
+
+R, C = 70, 1024
+
+
+def test_a_result_over_an_operand_that_every_row_reads():
+    """relu(x + v) stored over memory that holds v: one step after the other, v has been read by then."""
+    ops = [("Add", [_tensor(0, R, C), _tensor(1, C)], _tensor(2, R, C)), ("ReLU", [_tensor(2, R, C)], _tensor(3, R, C))]
+    exe = api.GraphCompiler().compile(_partition(ops, [0, 1], [3]))
+    g = torch.Generator(device=DEV).manual_seed(1)
+    for row in (0, R // 2, R - 1):
+        x, out = _bf(g, R, C), _bf(g, R, C)
+        v = out[row]
+        want = torch.relu(x + v)
+        exe.execute_on_stream({0: x, 1: v}, {3: out})
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+
+
+def test_a_row_result_in_place_of_a_row_operand():
+    """s = row + one value, stored in place of row, and x * s: no part of a row may see the new value as the old one."""
+    ops = [("Add", [_floats(0, R, 1), _floats(1, 1)], _floats(2, R, 1)), ("Multiply", [_floats(3, R, C), _floats(2, R, 1)], _floats(4, R, C))]
+    exe = api.GraphCompiler().compile(_partition(ops, [0, 1, 3], [2, 4]))
+    g = torch.Generator(device=DEV).manual_seed(2)
+    row, one, x = (torch.randn(*s, generator=g, device=DEV) for s in ((R, 1), (1,), (R, C)))
+    s, out = row + one, torch.empty_like(x)
+    exe.execute_on_stream({0: row, 1: one, 3: x}, {2: row, 4: out})
+    torch.cuda.synchronize()
+    assert torch.equal(row, s) and torch.equal(out, x * s)
+
+
+def test_a_result_in_the_place_of_an_operand_of_its_shape():
+    """out = (x + y) * v over x: element by element, so the run stays one kernel."""
+    ops = [("Add", [_tensor(0, R, C), _tensor(1, R, C)], _tensor(2, R, C)), ("Multiply", [_tensor(2, R, C), _tensor(3, C)], _tensor(4, R, C))]
+    exe = api.GraphCompiler().compile(_partition(ops, [0, 1, 3], [4]))
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x, y, v = _bf(g, R, C), _bf(g, R, C), _bf(g, C)
+    want, n = (x + y) * v, lib.launch_count()
+    exe.execute_on_stream({0: x, 1: y, 3: v}, {4: x})
+    torch.cuda.synchronize()
+    assert torch.equal(x, want) and lib.launch_count() - n == 1
