@@ -452,14 +452,19 @@ Plan build_plan(Partition part) {
   }
 
   // ---- elementwise steps run together where they can (rowprog.h): a matmul that does not need the elementwise steps
-  // ahead of it moves in front of them, so that runs interrupted by one become whole
+  // ahead of it moves in front of them, so that runs interrupted by one become whole.  Only past and with results that the
+  // arena holds: results of the partition lie in the caller's buffers, which may share memory with an argument that a step
+  // further ahead has still to read.
   auto elementwise = [](const Step &st) {
     return st.kind == StepKind::BINARY || st.kind == StepKind::UNARY || st.kind == StepKind::REDUCE;
   };
   for (size_t i = 1; i < plan.steps.size(); ++i) {
     if (plan.steps[i].kind != StepKind::MATMUL && plan.steps[i].kind != StepKind::QMATMUL) continue;
     size_t j = i;
+    auto leaves = [&](size_t id) { return std::find(p.output_ids.begin(), p.output_ids.end(), id) != p.output_ids.end(); };
+    if (std::any_of(plan.steps[i].out.begin(), plan.steps[i].out.end(), leaves)) continue;
     auto independent = [&](const Step &before) {
+      if (std::any_of(before.out.begin(), before.out.end(), leaves)) return false;
       for (size_t id : before.out)
         if (std::find(plan.steps[i].in.begin(), plan.steps[i].in.end(), id) != plan.steps[i].in.end()) return false;
       return elementwise(before);

@@ -282,6 +282,26 @@ def test_tile_selection_for_the_benchmark_shapes():
         assert 16 <= c.bn <= 256 and c.bn % 16 == 0 and 2 <= c.stages <= 8 and c.splits >= 1 and c.grid >= 1
 
 
+@pytest.mark.parametrize("leaving", [(), ("sigmoid",), ("product",)])
+def test_matmuls_move_only_among_results_of_the_arena(leaving):
+    """The second product needs nothing of the sigmoid ahead of it and moves in front, so that the elementwise steps run
+    together - unless either result is the caller's, whose buffer may be the memory of an argument that is still to be read."""
+    t = lambda i, *s: {"id": i, "dtype": "bf16", "shape": list(s)}
+    graph = [{"kind": "Sigmoid", "inputs": [t(0, 128, 64)], "outputs": [t(4, 128, 64)]},
+             {"kind": "MatMul", "inputs": [t(1, 128, 64), t(2, 64, 64)], "outputs": [t(5, 128, 64)]},
+             {"kind": "Sigmoid", "inputs": [t(5, 128, 64)], "outputs": [t(6, 128, 64)]},
+             {"kind": "MatMul", "inputs": [t(1, 128, 64), t(3, 64, 64)], "outputs": [t(7, 128, 64)]},
+             {"kind": "Multiply", "inputs": [t(6, 128, 64), t(7, 128, 64)], "outputs": [t(8, 128, 64)]},
+             {"kind": "Multiply", "inputs": [t(8, 128, 64), t(4, 128, 64)], "outputs": [t(9, 128, 64)]}]
+    outs = [9] + [{"sigmoid": 6, "product": 7}[k] for k in leaving]
+    js = json.dumps({"version": "3.5.0", "engine_kind": "cpu", "fpmath_mode": "any", "input_ports": [0, 1, 2, 3], "output_ports": outs, "graph": graph})
+    plan = api.GraphCompiler().compile(js).plan()
+    kinds = re.findall(r"^step \d+: (\w+)", plan, re.M)
+    moved = ["Sigmoid", "MatMul", "MatMul", "Sigmoid", "Multiply", "Multiply"]
+    stays = ["Sigmoid", "MatMul", "Sigmoid", "MatMul", "Multiply", "Multiply"]
+    assert kinds == (stays if leaving else moved), plan
+
+
 class _Lent:
     """An object with a buffer and a shape that is neither a tensor nor an array."""
     shape = (8, 8)
