@@ -466,8 +466,11 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   p.a = operand_geom(a_mn, 128, eb, kpb);
   p.b = operand_geom(b_mn, pair ? p.BN / 2 : p.BN, eb, kpb);
   p.idesc = umma_instr_desc(a.int8 ? 2u : 1u, fa, fb, a_mn ? 1u : 0u, b_mn ? 1u : 0u, pair ? 256u : 128u, uint32_t(p.BN));
+  // Two accumulators.  The row-major epilogues read whole slabs of 64 (bf16) or 32 columns, so the last slab of the second
+  // one may reach beyond its BN columns (a 32-wide bf16 tile: columns 32 to 95) and must still lie in what is allocated.
+  const int slab = a.out_kind == OUT_BF16 ? 64 : 32, reach = cfg.swapped ? 2 * p.BN : p.BN + ceil_div(p.BN, slab) * slab;
   uint32_t cols = 32;
-  while (cols < uint32_t(2 * p.BN)) cols <<= 1;
+  while (cols < uint32_t(reach)) cols <<= 1;
   p.tmem_cols = cols;
 
   const CUtensorMap tmA = operand_tmap(p.a, ta, eb, pa, mn_a, a.K, 128, kpb, ld_a);

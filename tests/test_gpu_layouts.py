@@ -44,6 +44,24 @@ def test_bf16_layouts_without_alignment(M, N, K, ta, tb, bias, relu, skip):
     assert_bf16_close(tbits(Y), want, K, what=f"{M}x{N}x{K}", pre=acc if bias else None)
 
 
+@pytest.mark.parametrize("bn", [32, 96, 160])
+@pytest.mark.parametrize("M,N,K,tb", [(130, 131, 200, 0), (300, 193, 129, 1), (129, 320, 64, 0)])
+def test_recorded_tile_widths_of_no_whole_slab(M, N, K, tb, bn):
+    """Tiles whose last 64-column slab reaches beyond the accumulator, with results the copy engine cannot store (N odd) and
+    with results it can."""
+    A, B, b = (_rand(s, i).bfloat16() for i, s in enumerate([(M, K), (K, N), (N,)]))
+    lib.tune_cache_put(M, N, K, lib.MatmulConfig(0, bn, 1, 4, 8, 148, 0, 1))
+    try:
+        Y = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        lib.matmul_bf16(A.to(DEV), (B.t().contiguous() if tb else B).to(DEV), b.to(DEV), True, False, bool(tb), out=Y)
+        torch.cuda.synchronize()
+    finally:
+        lib.tune_cache_erase(M, N, K)
+    assert lib.device_error() == 0
+    want, acc = oracle.linear_bf16(tbits(A), tbits(B), tbits(b), relu=True, return_acc=True)
+    assert_bf16_close(tbits(Y), want, K, what=f"{M}x{N}x{K} tile {bn}", pre=acc)
+
+
 @pytest.mark.parametrize("M,N,K,ta,tb", [(700, 1300, 40, 0, 0), (65, 66, 17, 1, 0), (40, 130, 33, 0, 1), (5, 768, 100, 0, 0), (17, 31, 16, 1, 1),
                                          (640, 1024, 16, 1, 1), (1, 1, 1, 0, 0)])
 def test_f32_bits(M, N, K, ta, tb):
