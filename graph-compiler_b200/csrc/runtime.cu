@@ -139,6 +139,7 @@ MatmulConfig select_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_byt
   MatmulConfig c{};
   if (!std::getenv("GC_B200_TILE") && tune::lookup(tune::Key{M, N, K, dtype_bytes, out_bytes}, &c) && (!c.swapped || M <= 64)) {
     if (c.grid <= 0 || c.grid > sm_count) c.grid = sm_count;
+    c.chosen = 7;
     return c;
   }
   return model_matmul_config(M, N, K, dtype_bytes, out_bytes, sm_count);
@@ -262,6 +263,7 @@ MatmulConfig model_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_byte
       if (sp > 0) { const int per = ceil_div(k_blocks, sp); c.splits = ceil_div(k_blocks, per); }
       if (st > 0) c.stages = std::min(st, c.stages);
       if (gm > 0) c.group_m = gm;
+      c.chosen = (sp > 0 ? 1 : 0) | (st > 0 ? 2 : 0) | (kp > 0 ? 4 : 0);
       const int t2 = c.swapped ? ceil_div(N, 128) : ceil_div(M, 128) * ceil_div(N, c.bn);
       c.grid = std::min(t2 * c.splits, sm_count);
     }
@@ -279,37 +281,41 @@ size_t matmul_scratch_bytes(int64_t M, int64_t N, int64_t K, int dtype_bytes, in
 // the others, the weights arrive at 7.5 TB/s at best, and handing parts round the cluster costs 1 us and 0.06 us for every row
 // that a CTA finishes: the split with the cheapest sum over the rounds.  Fitted to eighteen shapes from 300 x 1100 to
 // 28672 x 8192 with 1, 16, 32 and 64 rows, every split timed: 1.4 % behind the best one on average.
-static int decode_split(int tiles, int k_blocks, int kpb, int64_t rows, bool int8, int device, int *at_once) {
-  int best = 1;
+FewRowsPlan plan_few_rows(int64_t M, int64_t N, int64_t K, bool int8, const MatmulConfig &cfg, int sm_count, int device) {
+  const int k_blocks = ceil_div(K, int8 ? 128 : 64);
+  FewRowsPlan r{ceil_div(N, 128), 1, k_blocks >= 2 ? 2 : 1, 1};
+  if (cfg.chosen & 4) r.kpb = std::min(r.kpb, std::max(1, cfg.kpb));
+  const int most = (cfg.chosen & 1) ? std::max(1, std::min(8, cfg.splits)) : 8;
   double best_t = 1e30;
-  for (int split = 1; split <= 8; ++split) {
-    const int per = ceil_div(ceil_div(k_blocks, split), kpb) * kpb;
+  for (int split = most; split >= 1; --split) {
+    const int per = ceil_div(ceil_div(k_blocks, split), r.kpb) * r.kpb;
     if (split > 1 && per * (split - 1) >= k_blocks) continue;   // the last CTA would have nothing to do
-    const int clusters = decode_clusters_at_once(int8, device, split);
+    const int clusters = device < 0 ? sm_count / split : decode_clusters_at_once(int8, device, split);
     if (clusters < 1) continue;
-    const int rounds = ceil_div(tiles, clusters), active = std::min(tiles, clusters) * split;
-    const double stream = double(tiles) * k_blocks * 16384 / 7.5e6;
-    const double t = std::max(stream, rounds * per * std::max(0.17, active * 16384 / 7.5e6)) + (split > 1 ? rounds * (1.0 + 0.06 * double(rows) / split) : 0.0);
-    if (t < best_t) {
+    const int rounds = ceil_div(r.tiles, clusters), active = std::min(r.tiles, clusters) * split;
+    const double stream = double(r.tiles) * k_blocks * 16384 / 7.5e6;
+    const double t = std::max(stream, rounds * per * std::max(0.17, active * 16384 / 7.5e6)) + (split > 1 ? rounds * (1.0 + 0.06 * double(M) / split) : 0.0);
+    if (t <= best_t) {
       best_t = t;
-      best = split;
-      *at_once = clusters;
+      r.split = split;
+      r.clusters = clusters;
     }
+    if (cfg.chosen & 1) break;   // as recorded, or the next smaller one that runs
   }
-  return best;
+  return r;
 }
 
-static void matmul_decode(const MatmulArgs &a, cudaStream_t stream) {
+static void matmul_decode(const MatmulArgs &a, const MatmulConfig &cfg, cudaStream_t stream) {
   DeviceState &dev = device_state();
   const int eb = a.int8 ? 1 : 2;
   DecodeParams p{};
   const bool w_mn = a.trans_b == 0, x_mn = a.trans_a != 0;
   p.bk_elems = 128 / eb;
   p.k_blocks = ceil_div(a.K, p.bk_elems);
-  p.tiles = ceil_div(a.N, 128);
-  int clusters = 1;
-  p.kpb = p.k_blocks >= 2 ? 2 : 1;
-  p.split = decode_split(p.tiles, p.k_blocks, p.kpb, a.M, a.int8 != 0, dev.device, &clusters);
+  const FewRowsPlan plan = plan_few_rows(a.M, a.N, a.K, a.int8 != 0, cfg, dev.sm_count, dev.device);
+  p.tiles = plan.tiles;
+  p.kpb = plan.kpb;
+  p.split = plan.split;
   p.parts_bytes = p.split > 1 ? uint32_t(a.M) * 512u : 0u;
   p.BN = std::max(16, ceil_div(a.M, 16) * 16);
   p.early_weights = a.early_weights || a.early_inputs;
@@ -321,6 +327,7 @@ static void matmul_decode(const MatmulArgs &a, cudaStream_t stream) {
   p.tmem_cols = 32;
   while (p.tmem_cols < uint32_t(2 * p.BN)) p.tmem_cols <<= 1;
   p.stages = decode_stages(p);
+  if (cfg.chosen & 2) p.stages = std::min(p.stages, std::max(2, cfg.stages));
   p.out_kind = a.out_kind;
   p.out = a.out;
   p.ld_out = a.ld_out ? a.ld_out : a.N;
@@ -334,7 +341,7 @@ static void matmul_decode(const MatmulArgs &a, cudaStream_t stream) {
   p.out_rows = int(a.M);
   p.out_cols = int(a.N);
   p.error = dev.d_error;
-  const int grid = std::min(p.tiles, clusters) * p.split;
+  const int grid = std::min(p.tiles, plan.clusters) * p.split;
   cudaError_t e = a.int8 ? launch_gemm_decode<1>(tmW, tmX, p, grid, dev.device, stream) : launch_gemm_decode<0>(tmW, tmX, p, grid, dev.device, stream);
   if (e != cudaSuccess) throw CudaError(std::string("few-rows gemm launch: ") + cudaGetErrorString(e));
   count_launch();
@@ -412,7 +419,7 @@ void matmul_tc(const MatmulArgs &a, cudaStream_t stream) {
   MatmulConfig cfg = a.force ? *a.force : select_matmul_config(a.M, a.N, a.K, eb, out_bytes, dev.sm_count, max_splits);
   const int64_t ld_out = a.ld_out ? a.ld_out : a.N;
   if (cfg.swapped && !a.force && a.n_peers == 0 && !a.wait_counter && !a.trace) {
-    matmul_decode(a, stream);
+    matmul_decode(a, cfg, stream);
     return;
   }
 

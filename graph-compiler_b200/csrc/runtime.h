@@ -71,7 +71,19 @@ struct MatmulConfig {
   int grid;      // CTAs launched (persistent)
   int pair;      // 1: CTA-pair kernel (256 x bn tiles, two SMs per tile)
   int kpb;       // K blocks of 128 bytes per pipeline stage (0 or 1: one)
+  // Fields that were recorded or overridden and not left to the model (host only): 1 splits, 2 stages, 4 kpb.  The few-rows
+  // kernel, which has a rule of its own, follows these.
+  int chosen = 0;
 };
+// How the few-rows kernel shares out a matmul whose configuration is `swapped`.
+struct FewRowsPlan {
+  int tiles;      // of 128 output columns
+  int split;      // CTAs of a cluster, which share a tile's K range
+  int kpb;        // K blocks of a stage
+  int clusters;   // at the same time
+};
+// device < 0: without asking one; clusters are then as many as sm_count allows.
+FewRowsPlan plan_few_rows(int64_t M, int64_t N, int64_t K, bool int8, const MatmulConfig &cfg, int sm_count, int device);
 // dtype_bytes: 2 (bf16) or 1 (int8).  out_bytes: bytes per output element written by the GEMM kernel.
 // max_splits < 8 restricts the K split (1: none - launches whose partial sums leave through peer stores); such a
 // request is answered by the model alone.

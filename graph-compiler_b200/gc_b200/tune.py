@@ -21,7 +21,8 @@ from . import lib
 
 def candidates(M: int, N: int, K: int, dtype_bytes: int = 2, out_bytes: int = 2, sms: int = 148) -> List[lib.MatmulConfig]:
     """The model's configuration first, then its neighbours: tile widths, K splits and K blocks per stage
-    that the kernels accept for this shape.  Pure host logic."""
+    that the kernels accept for this shape.  For few rows (``swapped``) a K split is the number of CTAs that share a
+    tile's K range.  Pure host logic."""
     base = lib.model_matmul_config(M, N, K, dtype_bytes, out_bytes, sms)
     k_blocks = -(-K // (128 // dtype_bytes))
     out: List[lib.MatmulConfig] = [base]
@@ -83,7 +84,10 @@ def tune_matmul(M: int, N: int, K: int, int8: bool = False, iters: int = 10, rec
     """Times every candidate for a bf16 (or u8 x s8, dequantised f32) matmul of this shape on the current device.
     Returns (best configuration, its microseconds, [(repr, microseconds or nan)] for all candidates); records the
     best one in the measured-configuration cache unless ``record`` is False.  Inputs smaller than 256 MB are timed
-    with a write of a 256 MiB buffer between launches so that operands come from HBM."""
+    with a write of a 256 MiB buffer between launches so that operands come from HBM.
+
+    With few rows the kernel shares K out by a rule of its own unless a configuration is recorded; that rule is what
+    the first candidate stands for, and where it is not beaten nothing is recorded."""
     import torch
 
     dev = torch.device("cuda", torch.cuda.current_device())
@@ -103,12 +107,16 @@ def tune_matmul(M: int, N: int, K: int, int8: bool = False, iters: int = 10, rec
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev) if (M * K + K * N) * eb + M * N * ob < 256e6 else None
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     cands = list(configs) if configs is not None else candidates(M, N, K, eb, ob, sms)
+    own_rule = configs is None and cands[0].swapped
     results, best, best_us = [], None, float("inf")
     saved = lib.tune_cache_get(M, N, K, eb, ob)
     try:
-        for c in cands:
+        for i, c in enumerate(cands):
             try:
-                lib.tune_cache_put(M, N, K, c, eb, ob)     # the launchers pick the recorded configuration up
+                if own_rule and i == 0:
+                    lib.tune_cache_erase(M, N, K, eb, ob)
+                else:
+                    lib.tune_cache_put(M, N, K, c, eb, ob)     # the launchers pick the recorded configuration up
                 us = _time(run, iters, flush)
             except RuntimeError:                           # a candidate the kernels reject (shared memory, alignment)
                 us = float("nan")
@@ -123,7 +131,10 @@ def tune_matmul(M: int, N: int, K: int, int8: bool = False, iters: int = 10, rec
         else:
             lib.tune_cache_erase(M, N, K, eb, ob)
     if best is not None and record:
-        lib.tune_cache_put(M, N, K, best, eb, ob)
+        if own_rule and best is cands[0]:
+            lib.tune_cache_erase(M, N, K, eb, ob)
+        else:
+            lib.tune_cache_put(M, N, K, best, eb, ob)
     return best, best_us, results
 
 

@@ -168,7 +168,10 @@ int gcb200_select_matmul_config(int64_t M, int64_t N, int64_t K, int dtype_bytes
  * device, see gc_b200/tune.py) takes precedence over the model in gcb200_select_matmul_config and in every
  * matmul launch of that exact shape; the cache is a text file (one "M N K dtype_bytes out_bytes : swapped bn
  * splits stages group_m grid pair kpb" line per shape), read once from the path in GC_B200_TUNE_CACHE and
- * loadable / savable explicitly.  The reference's counterpart is the per-op override attribute set of
+ * loadable / savable explicitly.  Few rows (`swapped`: at most 64 rows, 128 columns and more) run on a kernel that
+ * shares a tile's K range among the CTAs of a cluster by a rule of its own; a recorded configuration (or GC_B200_TILE)
+ * sets it instead: splits = CTAs per cluster (at most 8), kpb, stages.  The model's `splits` for these shapes is that
+ * of gcb200_matmul_bf16_cfg, which runs the tile kernel.  The reference's counterpart is the per-op override attribute set of
  * MatmulConfigAnalysis.cpp:368-401.  Host logic; needs no device. */
 int gcb200_tune_cache_put(int64_t M, int64_t N, int64_t K, int dtype_bytes, int out_bytes, const gcb200_matmul_config *cfg);
 int gcb200_tune_cache_get(int64_t M, int64_t N, int64_t K, int dtype_bytes, int out_bytes, gcb200_matmul_config *cfg, int *found);

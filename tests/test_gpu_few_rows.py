@@ -98,3 +98,33 @@ torch.save([x.cpu() for x in o], sys.argv[1])
 ])
 def test_few_rows_stages_of_two_k_blocks(M, N, K, tb):
     test_few_rows_match_the_oracle_every_time(M, N, K, 0, tb)
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 512, 8192), (33, 1040, 1096), (64, 4096, 520), (1, 130, 136)])
+def test_few_rows_as_recorded(M, N, K):
+    """Every share of K, one and two K blocks to a stage and short rings, set by a recorded configuration."""
+    g = torch.Generator().manual_seed(M + K)
+    A, B, b = ((torch.rand(s, generator=g) * 2 - 1).bfloat16() for s in ((M, K), (K, N), (N,)))
+    Ad, Bd, bd = A.to(DEV), B.to(DEV), b.to(DEV)
+    want, acc = oracle.linear_bf16(tbits(A), tbits(B), tbits(b), relu=True, return_acc=True)
+    try:
+        for splits, kpb, stages in [(1, 1, 2), (2, 2, 3), (3, 1, 8), (5, 2, 2), (7, 1, 5), (8, 2, 8), (64, 4, 8)]:
+            lib.tune_cache_put(M, N, K, lib.MatmulConfig(1, 64, splits, stages, 8, 148, 0, kpb))
+            Y = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+            lib.matmul_bf16(Ad, Bd, bd, True, out=Y)
+            torch.cuda.synchronize()
+            assert lib.device_error() == 0
+            assert_bf16_close(tbits(Y), want, K, what=f"{M}x{N}x{K} clusters of {splits}, {kpb} blocks, {stages} stages", pre=acc)
+    finally:
+        lib.tune_cache_erase(M, N, K)
+
+
+def test_tuning_few_rows_records_only_what_beats_the_own_rule():
+    from gc_b200 import tune
+
+    M, N, K = 16, 1024, 8192
+    best, us, results = tune.tune_matmul(M, N, K, iters=3)
+    assert len(results) > 4 and all(t > 0 for _, t in results)
+    recorded = lib.tune_cache_get(M, N, K)
+    lib.tune_cache_erase(M, N, K)
+    assert (recorded is None) == (repr(best) == results[0][0])
