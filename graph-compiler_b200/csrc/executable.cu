@@ -457,11 +457,20 @@ struct dnnl_graph_compiler_executable {
     return bad;
   }
 
-  // One line per step with the kernel and, for matmuls, the tile configuration the selector gives for `sm_count` SMs.
+  // One line per step with the kernel and, for matmuls, the tile configuration the selector gives for `sm_count` SMs; for the
+  // few-rows kernel what it makes of it (on the device at hand if that has as many SMs, else without asking one).
   std::string describe_launches(int sm_count) const {
+    int on = -1;
+    try {
+      if (device_state().sm_count == sm_count) on = device_state().device;
+    } catch (const CudaError &) {
+    }
     std::ostringstream os;
+    int run = -1;   // the elementwise run that step i belongs to
     for (size_t i = 0; i < plan.steps.size(); ++i) {
       const Step &st = plan.steps[i];
+      if (group_at[i] >= 0) run = group_at[i];
+      if (run >= 0 && size_t(groups[size_t(run)].last) < i) run = -1;
       os << "  step " << i << " " << st.op << ": ";
       if (st.kind == StepKind::MATMUL || st.kind == StepKind::QMATMUL) {
         const bool q = st.kind == StepKind::QMATMUL;
@@ -472,11 +481,21 @@ struct dnnl_graph_compiler_executable {
         }
         const bool tma = (st.trans_a ? st.M : st.K) % 8 == 0 && (st.trans_b ? st.K : st.N) % 8 == 0;
         const MatmulConfig c = select_matmul_config(st.M, st.N, st.K, q ? 1 : 2, q ? 4 : 2, sm_count);
-        os << "gemm_kernel<" << (q ? "u8 x s8" : "bf16") << (c.swapped ? ", weights on the MMA M side" : "") << "> " << st.M << "x" << st.N
-           << "x" << st.K << " tile 128x" << c.bn << " splits " << c.splits << " stages " << c.stages << " K blocks/stage "
-           << std::max(1, c.kpb) << " grid " << c.grid << (!q && !tma ? " + pack_rows" : "") << (c.splits > 1 ? " + reduce_planes" : "") << (q ? " + colsum_s8" : "") << "\n";
+        const std::string around = std::string(!q && !tma ? " + pack_rows" : "") + (q && st.zp_a != 0 ? " + colsum_s8" : "");
+        if (c.swapped) {
+          const FewRowsPlan f = plan_few_rows(st.M, st.N, st.K, q, c, sm_count, on);
+          os << "gemm_decode_kernel<" << (q ? "u8 x s8" : "bf16") << "> " << st.M << "x" << st.N << "x" << st.K << " tiles of 128 columns " << f.tiles
+             << " clusters of " << f.split << " K blocks/stage " << f.kpb << " grid " << std::min(f.tiles, f.clusters) * f.split << around << "\n";
+          continue;
+        }
+        os << "gemm_kernel<" << (q ? "u8 x s8" : "bf16") << "> " << st.M << "x" << st.N << "x" << st.K << " tile 128x" << c.bn << " splits " << c.splits << " stages " << c.stages << " K blocks/stage " << std::max(1, c.kpb)
+           << " grid " << c.grid << (c.pair ? " on CTA pairs" : "") << (c.splits <= 1 ? "" : defers[i] ? ", partial sums added by the run that reads them" : " + reduce_planes") << around << "\n";
       } else if (st.kind == StepKind::SDPA) {
         os << "attention_kernel B*H=" << st.batch * st.heads << " S=" << st.seq << " D=" << st.dim << " causal=" << st.causal << "\n";
+      } else if (run >= 0 && size_t(groups[size_t(run)].first) < i) {
+        os << "in the kernel of step " << groups[size_t(run)].first << "\n";
+      } else if (run >= 0) {
+        os << "row_program_kernel, steps " << groups[size_t(run)].first << " to " << groups[size_t(run)].last << "\n";
       } else {
         os << (st.kind == StepKind::REDUCE ? "reduce kernel" : st.kind == StepKind::BINARY ? "binary_kernel"
                : st.kind == StepKind::COPY ? "device-to-device copy" : "unary_kernel") << "\n";

@@ -302,6 +302,39 @@ def test_matmuls_move_only_among_results_of_the_arena(leaving):
     assert kinds == (stays if leaving else moved), plan
 
 
+def test_few_rows_follow_a_recorded_configuration_and_launches_say_so(monkeypatch):
+    """Plain launches of at most 64 rows run the few-rows kernel: what is recorded or overridden is what it does, and the launch
+    list names it with the split that runs."""
+    clusters = lambda M, N, K: tuple(int(v) for v in re.search(
+        r"gemm_decode_kernel<bf16> %dx%dx%d tiles of 128 columns \d+ clusters of (\d+) K blocks/stage (\d+)" % (M, N, K),
+        api.GraphCompiler().compile(partitions.matmul(M, N, K)[0]).launches()).groups())
+    lib.tune_cache_clear()
+    try:
+        own = clusters(16, 512, 8192)
+        assert own[0] > 1 and own[1] == 2
+        lib.tune_cache_put(16, 512, 8192, lib.MatmulConfig(1, 16, 3, 4, 8, 148, 0, 1))
+        assert clusters(16, 512, 8192) == (3, 1)
+        lib.tune_cache_put(16, 512, 8192, lib.MatmulConfig(1, 16, 32, 4, 8, 148, 0, 2))   # more than a cluster holds
+        assert clusters(16, 512, 8192) == (8, 2)
+        lib.tune_cache_put(16, 512, 256, lib.MatmulConfig(1, 16, 8, 4, 8, 148, 0, 2))     # two CTAs have a whole stage each
+        assert clusters(16, 512, 256) == (2, 2)
+        lib.tune_cache_clear()
+        assert clusters(16, 512, 8192) == own
+        monkeypatch.setenv("GC_B200_TILE", "0,5")
+        assert clusters(16, 512, 8192) == (5, 2)
+        monkeypatch.setenv("GC_B200_TILE", "128,0,0,4")   # nothing that this kernel has
+        assert clusters(16, 512, 8192) == own
+    finally:
+        lib.tune_cache_clear()
+
+
+def test_launches_name_fused_runs_and_leave_out_what_does_not_run():
+    text = api.GraphCompiler().compile(partitions.llama2_mlp(1, 128, 512, 1024)[0]).launches()
+    assert re.search(r"step 1 Add: row_program_kernel, steps 1 to 9\n  step 2 Typecast: in the kernel of step 1\n", text), text
+    assert "colsum_s8" not in api.GraphCompiler().compile(partitions.quantized_matmul(128, 256, 256, 0)[0]).launches()
+    assert "colsum_s8" in api.GraphCompiler().compile(partitions.quantized_matmul(128, 256, 256, 3)[0]).launches()
+
+
 class _Lent:
     """An object with a buffer and a shape that is neither a tensor nor an array."""
     shape = (8, 8)
