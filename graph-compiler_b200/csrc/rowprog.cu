@@ -1,6 +1,7 @@
 #include "rowprog.h"
 
 #include <algorithm>
+#include <mutex>
 #include <stdexcept>
 #include <unordered_map>
 
@@ -11,21 +12,6 @@ namespace gcb {
 
 // ----------------------------------------------------------------------------- kernel
 namespace {
-
-template <int N> __device__ __forceinline__ void fetch(const float (&v)[kProgRegs][kProgVec], const float (&s)[kProgRowRegs], int r, float (&x)[N]) {
-#pragma unroll
-  for (int k = 0; k < kProgRegs; ++k)
-    if (r == k) {
-#pragma unroll
-      for (int e = 0; e < N; ++e) x[e] = v[k][e];
-    }
-#pragma unroll
-  for (int k = 0; k < kProgRowRegs; ++k)
-    if (r == 16 + k) {
-#pragma unroll
-      for (int e = 0; e < N; ++e) x[e] = s[k];
-    }
-}
 
 __device__ __forceinline__ void load8(const void *p, long long i, int dt, float (&x)[kProgVec]) {
   if (dt == 0) {
@@ -59,15 +45,71 @@ __device__ __forceinline__ void store8(void *p, long long i, int dt, const float
   *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p) + i) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Each thread carries eight consecutive values of a row in every vector register and a copy of the row's values in the
-// row registers.  With a reduction a block owns one row; without, blocks walk the tensor in 8-value chunks.  Registers
-// are named by the program, so an operand is picked by uniform branches; against the launches it replaces (2 to 3 us
-// each, nine of them for an RMSNorm) the interpretation - some hundred cycles per operation - does not show.
+// One choice for all eight values: chosen value by value, the branches were most of an operation.
+template <class F> __device__ __forceinline__ void each(float (&r)[kProgVec], F f) {
+#pragma unroll
+  for (int e = 0; e < kProgVec; ++e) r[e] = f(e);
+}
+__device__ __forceinline__ void binary8(int fn, const float (&x)[kProgVec], const float (&y)[kProgVec], float (&r)[kProgVec]) {
+  switch (fn) {
+  case 0: each(r, [&](int e) { return ew_binary(0, x[e], y[e]); }); break;
+  case 1: each(r, [&](int e) { return ew_binary(1, x[e], y[e]); }); break;
+  case 2: each(r, [&](int e) { return ew_binary(2, x[e], y[e]); }); break;
+  default: each(r, [&](int e) { return ew_binary(3, x[e], y[e]); }); break;
+  }
+}
+__device__ __forceinline__ void unary8(int fn, float beta, const float (&x)[kProgVec], float (&r)[kProgVec]) {
+  switch (fn) {
+  case 0: each(r, [&](int e) { return ew_unary(0, beta, x[e]); }); break;
+  case 1: each(r, [&](int e) { return ew_unary(1, beta, x[e]); }); break;
+  case 2:
+    if (beta == 2.f) each(r, [&](int e) { return ew_unary(2, 2.f, x[e]); });
+    else each(r, [&](int e) { return ew_unary(2, beta, x[e]); });
+    break;
+  case 4: each(r, [&](int e) { return ew_unary(4, beta, x[e]); }); break;
+  case 5: each(r, [&](int e) { return ew_unary(5, beta, x[e]); }); break;
+  default: each(r, [&](int e) { return x[e]; }); break;
+  }
+}
+__device__ __forceinline__ void round8(float (&r)[kProgVec], int dt) {
+  if (dt == 1) each(r, [&](int e) { return ew_round(r[e], 1); });
+  else if (dt == 2) each(r, [&](int e) { return ew_round(r[e], 2); });
+}
+
+// A thread's registers lie in shared memory, where the program can index them.  Picked from real registers by comparisons,
+// with a branch per value for the operation, one operation took a block some 2000 cycles, and at 128 registers a thread an SM
+// held one block of wide rows: x^2, mean, x * m^-0.5 * v over 2368 x 3072 bf16 134.8 us, where the steps one by one take 99;
+// in this form 40.0 (1.1 TB/s in and out).  9472 x 4096 560 -> 195 (steps: 571), add + relu over 16384 x 4096 421 -> 206, the
+// decoder block's runs with 32 tokens together 29 -> 11 us, with 512 tokens the block 354 -> 239.
+struct Registers {
+  float4 *v;   // [register][half][thread]
+  float *s;    // [register][thread]
+  __device__ __forceinline__ void get(int r, float (&x)[kProgVec]) const {
+    if (r >= 16) {
+      const float f = s[(r - 16) * blockDim.x];
+      each(x, [&](int) { return f; });
+      return;
+    }
+    const float4 a = v[(2 * r) * blockDim.x], b = v[(2 * r + 1) * blockDim.x];
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  }
+  __device__ __forceinline__ void set(int r, const float (&x)[kProgVec]) const {
+    v[(2 * r) * blockDim.x] = make_float4(x[0], x[1], x[2], x[3]);
+    v[(2 * r + 1) * blockDim.x] = make_float4(x[4], x[5], x[6], x[7]);
+  }
+  __device__ __forceinline__ float &row(int r) const { return s[(r - 16) * blockDim.x]; }
+};
+constexpr size_t kRegisterBytes = kProgRegs * kProgVec * 4 + kProgRowRegs * 4;   // of a thread
+
+// Each thread has eight consecutive values of a row in every vector register and a copy of the row's values in the row
+// registers.  With a reduction a block owns one row; without, blocks walk the tensor in 8-value chunks.
 // Measured on the decoder block with 32 rows: 21 launches in 79 us before, 3 in 10 us.
-constexpr int kRowThreads = 512, kFlatThreads = 128;   // 512: 128 registers a thread, none spilled
+constexpr int kRowThreads = 512, kFlatThreads = 128;
 template <bool REDUCE>
-__global__ void __launch_bounds__(REDUCE ? kRowThreads : kFlatThreads) row_program_kernel(const __grid_constant__ RowProgram p) {
+__global__ void __launch_bounds__(REDUCE ? kRowThreads : kFlatThreads, REDUCE ? 2 : 8) row_program_kernel(const __grid_constant__ RowProgram p) {
+  extern __shared__ float4 registers[];
   __shared__ float part[32];
+  const Registers reg = {registers + threadIdx.x, reinterpret_cast<float *>(registers + kProgRegs * 2 * blockDim.x) + threadIdx.x};
   pdl_wait();
   pdl_launch_dependents();
   const int chunks = p.cols / kProgVec;
@@ -79,58 +121,46 @@ __global__ void __launch_bounds__(REDUCE ? kRowThreads : kFlatThreads) row_progr
     const bool in = !REDUCE || chunk < chunks;
     const int col = chunk * kProgVec;
     const long long at = row * p.cols + col;
-    float v[kProgRegs][kProgVec], s[kProgRowRegs];
-#pragma unroll
-    for (int k = 0; k < kProgRegs; ++k)
-#pragma unroll
-      for (int e = 0; e < kProgVec; ++e) v[k][e] = 0.f;
-#pragma unroll
-    for (int k = 0; k < kProgRowRegs; ++k) s[k] = 0.f;
     for (int i = 0; i < p.n; ++i) {
       const RowOp o = p.op[i];
+      float x[kProgVec], y[kProgVec], r[kProgVec];
       if (o.row) {
-        float r = 0.f, x[1] = {0.f}, y[1] = {0.f};
+        float f = 0.f;
         if (o.kind == RowOp::LOAD) {
-          r = ew_load(p.ptr[o.ptr], o.mode == 4 ? row : 0, o.dtype);
+          f = ew_load(p.ptr[o.ptr], o.mode == 4 ? row : 0, o.dtype);
         } else if (o.kind == RowOp::STORE) {
-          fetch<1>(v, s, o.a, x);
-          if (col == 0) ew_store(p.ptr[o.ptr], row, o.dtype, x[0]);
+          if (col == 0) ew_store(p.ptr[o.ptr], row, o.dtype, reg.row(o.a));
           continue;
         } else if (o.kind == RowOp::REDUCE) {
-          float t[kProgVec];
-          fetch<kProgVec>(v, s, o.a, t);
           if (REDUCE) {
             float sum = 0.f;
+            if (in) {
+              reg.get(o.a, x);
 #pragma unroll
-            for (int e = 0; e < kProgVec; ++e) sum = __fadd_rn(sum, t[e]);
-            if (!in) sum = 0.f;
+              for (int e = 0; e < kProgVec; ++e) sum = __fadd_rn(sum, x[e]);
+            }
 #pragma unroll
             for (int w = 16; w > 0; w >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xFFFFFFFFu, sum, w));
             __syncthreads();   // the shared sums of an earlier reduction have been read
             if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
             __syncthreads();
             const int warps = blockDim.x / 32;
-            for (int w = 0; w < warps; ++w) r = w == 0 ? part[0] : __fadd_rn(r, part[w]);
-            if (o.fn) r = __fdiv_rn(r, float(p.cols));
+            for (int w = 0; w < warps; ++w) f = w == 0 ? part[0] : __fadd_rn(f, part[w]);
+            if (o.fn) f = __fdiv_rn(f, float(p.cols));
           }
         } else {
-          fetch<1>(v, s, o.a, x);
-          if (o.kind == RowOp::BINARY) fetch<1>(v, s, o.b, y);
-          r = o.kind == RowOp::BINARY ? ew_binary(o.fn, x[0], y[0]) : ew_unary(o.fn, o.beta, x[0]);
+          f = o.kind == RowOp::BINARY ? ew_binary(o.fn, reg.row(o.a), reg.row(o.b)) : ew_unary(o.fn, o.beta, reg.row(o.a));
         }
-        if (o.kind != RowOp::LOAD) r = ew_round(r, o.dtype);
-#pragma unroll
-        for (int k = 0; k < kProgRowRegs; ++k)
-          if (o.dst == 16 + k) s[k] = r;
-        continue;
-      }
-      float r[kProgVec];
-      if (o.kind == RowOp::STORE) {
-        fetch<kProgVec>(v, s, o.a, r);
-        if (in) store8(p.ptr[o.ptr], at, o.dtype, r);
+        if (o.kind != RowOp::LOAD) f = ew_round(f, o.dtype);
+        reg.row(o.dst) = f;
         continue;
       }
       if (!in) continue;
+      if (o.kind == RowOp::STORE) {
+        reg.get(o.a, r);
+        store8(p.ptr[o.ptr], at, o.dtype, r);
+        continue;
+      }
       if (o.kind == RowOp::LOAD || (o.kind == RowOp::LOAD_PLANES && p.planes[o.ptr] == 0)) {
         load8(p.ptr[o.ptr], o.mode == 3 ? col : at, o.dtype, r);
       } else if (o.kind == RowOp::LOAD_PLANES) {
@@ -138,31 +168,22 @@ __global__ void __launch_bounds__(REDUCE ? kRowThreads : kFlatThreads) row_progr
         const float *base = reinterpret_cast<const float *>(p.ptr[o.ptr]);
         load8(base, at, 0, r);
         for (int k = 1; k < p.planes[o.ptr]; ++k) {
-          float t[kProgVec];
-          load8(base + (long long)k * p.plane_stride[o.ptr], at, 0, t);
+          load8(base + (long long)k * p.plane_stride[o.ptr], at, 0, x);
 #pragma unroll
-          for (int e = 0; e < kProgVec; ++e) r[e] = __fadd_rn(r[e], t[e]);
+          for (int e = 0; e < kProgVec; ++e) r[e] = __fadd_rn(r[e], x[e]);
         }
-#pragma unroll
-        for (int e = 0; e < kProgVec; ++e) r[e] = ew_round(r[e], 1);
+        round8(r, 1);
       } else if (o.kind == RowOp::BINARY) {
-        float x[kProgVec], y[kProgVec];
-        fetch<kProgVec>(v, s, o.a, x);
-        fetch<kProgVec>(v, s, o.b, y);
-#pragma unroll
-        for (int e = 0; e < kProgVec; ++e) r[e] = ew_round(ew_binary(o.fn, x[e], y[e]), o.dtype);
+        reg.get(o.a, x);
+        reg.get(o.b, y);
+        binary8(o.fn, x, y, r);
+        round8(r, o.dtype);
       } else {
-        float x[kProgVec];
-        fetch<kProgVec>(v, s, o.a, x);
-#pragma unroll
-        for (int e = 0; e < kProgVec; ++e) r[e] = ew_round(ew_unary(o.fn, o.beta, x[e]), o.dtype);
+        reg.get(o.a, x);
+        unary8(o.fn, o.beta, x, r);
+        round8(r, o.dtype);
       }
-#pragma unroll
-      for (int k = 0; k < kProgRegs; ++k)
-        if (o.dst == k) {
-#pragma unroll
-          for (int e = 0; e < kProgVec; ++e) v[k][e] = r[e];
-        }
+      reg.set(o.dst, r);
     }
   }
 }
@@ -180,7 +201,14 @@ void launch_row_program(const RowProgram &p, cudaStream_t stream) {
     cfg.blockDim = dim3(kFlatThreads);
     cfg.gridDim = dim3(unsigned(std::min<long long>((total + kFlatThreads - 1) / kFlatThreads, (long long)device_state().sm_count * 16)));
   }
+  cfg.dynamicSmemBytes = cfg.blockDim.x * kRegisterBytes;
   cfg.stream = stream;
+  if (p.has_reduce) {   // rows of more than 2700 columns need more shared memory than a block has without asking
+    static std::once_flag configured[64];
+    std::call_once(configured[device_state().device & 63], [] {
+      GCB_CUDA(cudaFuncSetAttribute(row_program_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRowThreads * kRegisterBytes)));
+    });
+  }
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
