@@ -462,18 +462,15 @@ std::vector<RowGroup> plan_row_groups(const Plan &plan) {
   const int n = int(plan.steps.size());
   for (int i = 0; i < n; ++i) {
     if (!fusable_kind(plan.steps[size_t(i)])) continue;
-    int best = -1;
-    RowGroup g;
-    for (int e = i + 1; e < n && fusable_kind(plan.steps[size_t(e)]); ++e) {
+    int end = i;
+    while (end + 1 < n && fusable_kind(plan.steps[size_t(end) + 1])) ++end;
+    for (int e = end; e > i; --e) {   // the longest run that one program holds: mostly the first try
       Compiler c(plan, i, e);
-      if (c.run()) {
-        best = e;
-        g = std::move(c.g);
-      }
+      if (!c.run()) continue;
+      groups.push_back(std::move(c.g));
+      i = e;
+      break;
     }
-    if (best < 0) continue;
-    groups.push_back(std::move(g));
-    i = best;
   }
   return groups;
 }
