@@ -1,6 +1,6 @@
 // CUDA runtime: device state, tensor maps, tile selection, matmul launch
 // planning and the small helper kernels (split-K reduction + epilogue, int8
-// column sums, exact-order SIMT matmul).
+// column sums).
 #include "runtime.h"
 #include "gemm_decode.h"
 #include "tune_cache.h"

@@ -28,11 +28,11 @@ def _no_device_error():
     (256, 512, 192, 0, 1, 1, 0),     # transpose_b: K-major weights
     (192, 320, 256, 1, 0, 1, 1),     # transpose_a: MN-major activations
     (200, 328, 136, 0, 0, 1, 1),     # ragged in M, N and K
-    (50, 72, 40, 0, 0, 1, 1),        # smaller than one tile (swapped orientation)
-    (16, 512, 1024, 0, 0, 1, 1),     # decode-shaped: swapped + split-K
+    (50, 72, 40, 0, 0, 1, 1),        # smaller than one tile
+    (16, 512, 1024, 0, 0, 1, 1),     # decode-shaped: few rows, K shared by a cluster
     (48, 1024, 512, 0, 1, 0, 1),
     (1024, 1024, 1024, 0, 0, 1, 1),  # several waves of tiles
-    (130, 36, 100, 0, 0, 1, 0),      # rows not 16-byte aligned: exact-order SIMT path
+    (130, 36, 100, 0, 0, 1, 0),      # rows not 16-byte aligned: operands packed first
     (1, 8, 8, 0, 0, 0, 0),
 ])
 def test_matmul_bf16_matches_oracle(M, N, K, ta, tb, bias, relu):
